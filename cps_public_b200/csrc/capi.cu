@@ -77,6 +77,7 @@ struct Staging {
       pin[k] = nullptr;
     }
     bytes = 0;
+    NoCallPool keep;  // shared by every call
     for (int k = 0; k < 2; k++) {
       CK(cudaMallocHost(&pin[k], n));
       dev[k].alloc(n);
@@ -88,6 +89,8 @@ Staging &staging() {
   static Staging s;
   return s;
 }
+
+std::atomic<int> live_gauges{0};  // resident gauge fields
 
 // memcpy of large vectors split over host threads.
 void par_copy(void *dst, const void *src, size_t n) {
@@ -150,6 +153,7 @@ int cpsb_init(int device) {
 int cpsb_mem_info(unsigned long long *free_b, unsigned long long *total_b) {
   return guarded([&] {
     need_init();
+    trim_pool();  // memory that the library keeps between calls is free memory
     size_t f = 0, t = 0;
     CK(cudaMemGetInfo(&f, &t));
     if (free_b) *free_b = f;
@@ -208,6 +212,7 @@ int cpsb_gauge_load(cpsb_gauge *out, const double *u, const int dims[4], int ord
     G.recon_err = worst;
     G.recon_ok = worst < 1e-6;
     *out = h.release();
+    live_gauges++;
     return CPSB_OK;
   });
 }
@@ -221,6 +226,7 @@ int cpsb_gauge_free(cpsb_gauge h) {
     CK(cudaStreamSynchronize(ctx().stream));
     drop_solvers(&h->g);
     delete h;
+    if (live_gauges.fetch_sub(1) == 1) trim_pool();  // the last resident field
     return CPSB_OK;
   });
 }
@@ -281,6 +287,7 @@ int cpsb_dslash(cpsb_gauge h, const cpsb_dirac_params *p, double *out, const dou
     check_params(h, p);
     if (!out || !in || (cb != 0 && cb != 1) || (dag != 0 && dag != 1)) throw Error{CPSB_ERR_ARG, "bad argument"};
     cudaStream_t st = ctx().stream;
+    CallPool pool(st);
     Operator op(&h->g, *p, P64, 1);
     Field fi(P64, op.nsites()), fo(P64, op.nsites());
     upload(fi, &in, 1, op.geom, st);
@@ -296,6 +303,7 @@ int cpsb_matpc(cpsb_gauge h, const cpsb_dirac_params *p, double *out, const doub
     check_params(h, p);
     if (!out || !in || (dag != 0 && dag != 1)) throw Error{CPSB_ERR_ARG, "bad argument"};
     cudaStream_t st = ctx().stream;
+    CallPool pool(st);
     Operator op(&h->g, *p, P64, 1);
     Field fi(P64, op.nsites()), fo(P64, op.nsites());
     upload(fi, &in, 1, op.geom, st);
@@ -311,6 +319,7 @@ int cpsb_mdagm(cpsb_gauge h, const cpsb_dirac_params *p, double *out, const doub
     check_params(h, p);
     if (!out || !in) throw Error{CPSB_ERR_ARG, "null vector"};
     cudaStream_t st = ctx().stream;
+    CallPool pool(st);
     Operator op(&h->g, *p, P64, 1);
     Field fi(P64, op.nsites()), fo(P64, op.nsites());
     RedSlot rs;
@@ -332,6 +341,7 @@ int cpsb_dslash_ex(cpsb_gauge h, const cpsb_dirac_params *p, int precision, doub
     if (precision < CPSB_PREC_F64 || precision > CPSB_PREC_F16) throw Error{CPSB_ERR_ARG, "bad precision"};
     if (!out || !in || (cb != 0 && cb != 1) || (dag != 0 && dag != 1)) throw Error{CPSB_ERR_ARG, "bad argument"};
     cudaStream_t st = ctx().stream;
+    CallPool pool(st);
     Operator op(&h->g, *p, precision, 1);
     Field fi(precision, op.nsites()), fo(precision, op.nsites());
     upload(fi, &in, 1, op.geom, st);
@@ -349,6 +359,7 @@ int cpsb_mdagm_ex(cpsb_gauge h, const cpsb_dirac_params *p, int precision, doubl
     if (precision < CPSB_PREC_F64 || precision > CPSB_PREC_F16) throw Error{CPSB_ERR_ARG, "bad precision"};
     if (!out || !in) throw Error{CPSB_ERR_ARG, "null vector"};
     cudaStream_t st = ctx().stream;
+    CallPool pool(st);
     Operator op(&h->g, *p, precision, 1);
     Field fi(precision, op.nsites()), fo(precision, op.nsites());
     RedSlot rs;
@@ -369,6 +380,7 @@ int cpsb_mdagm_dev(cpsb_gauge h, const cpsb_dirac_params *p, double *out, const 
     check_params(h, p);
     if (!out || !in) throw Error{CPSB_ERR_ARG, "null vector"};
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx().stream;
+    CallPool pool(st);
     Operator op(&h->g, *p, P64, 1);
     Field fi(P64, op.nsites()), fo(P64, op.nsites());
     RedSlot rs;
@@ -392,6 +404,7 @@ int cpsb_dslash_multi_dev(cpsb_gauge h, const cpsb_dirac_params *p, int precisio
     if (nrhs < 1 || nrhs > MAX_RHS) throw Error{CPSB_ERR_ARG, "nrhs out of range"};
     if (!out || !in || (cb != 0 && cb != 1) || (dag != 0 && dag != 1)) throw Error{CPSB_ERR_ARG, "bad argument"};
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx().stream;
+    CallPool pool(st);
     Operator op(&h->g, *p, precision, nrhs);
     Field fi(precision, op.nsites()), fo(precision, op.nsites());
     CK(launch_pack(precision, fi.ptr(), in, op.geom, st));
@@ -411,6 +424,7 @@ int cpsb_mdagm_multi_dev(cpsb_gauge h, const cpsb_dirac_params *p, int precision
     if (nrhs < 1 || nrhs > MAX_RHS) throw Error{CPSB_ERR_ARG, "nrhs out of range"};
     if (!out || !in) throw Error{CPSB_ERR_ARG, "null vector"};
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx().stream;
+    CallPool pool(st);
     Operator op(&h->g, *p, precision, nrhs);
     Field fi(precision, op.nsites()), fo(precision, op.nsites());
     RedSlot rs;
@@ -492,6 +506,7 @@ int cpsb_minvcg(cpsb_gauge h, const cpsb_dirac_params *p, const cpsb_cg_arg *a, 
     for (int i = 0; i < nvec; i++)
       if (!x[i]) throw Error{CPSB_ERR_ARG, "null solution vector"};
     cudaStream_t st = ctx().stream;
+    CallPool pool(st);
     const long n = cb_sites(h, p);
     const Geom g1 = geom_of(h, p, 1);
     Field chi(P64, n);
@@ -524,6 +539,7 @@ int cpsb_minvcg_dev(cpsb_gauge h, const cpsb_dirac_params *p, const cpsb_cg_arg 
     for (int i = 0; i < nvec; i++)
       if (!x[i]) throw Error{CPSB_ERR_ARG, "null solution vector"};
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx().stream;
+    CallPool pool(st);
     const long n = cb_sites(h, p);
     const Geom g1 = geom_of(h, p, 1);
     Field chi(P64, n);
@@ -565,6 +581,7 @@ int cpsb_minvcg_multi(cpsb_gauge h, const cpsb_dirac_params *p, const cpsb_cg_ar
     for (int q = 0; q < nvec; q++)
       if (!b[q]) throw Error{CPSB_ERR_ARG, "null source vector"};
     cudaStream_t st = ctx().stream;
+    CallPool pool(st);
     const long n1 = cb_sites(h, p);
     const Geom g1 = geom_of(h, p, 1);
     Field chi(P64, n1 * nvec);
@@ -596,6 +613,7 @@ int cpsb_minvcg_multi_dev(cpsb_gauge h, const cpsb_dirac_params *p, const cpsb_c
     for (int i = 0; i < nvec * nsol; i++)
       if (!x[i]) throw Error{CPSB_ERR_ARG, "null solution vector"};
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx().stream;
+    CallPool pool(st);
     const long n1 = cb_sites(h, p);
     const Geom g1 = geom_of(h, p, 1);
     Field chi(P64, n1 * nvec);
@@ -672,6 +690,7 @@ static int matinv_impl(cpsb_gauge h, const cpsb_dirac_params *p, const cpsb_cg_a
     if (zm && p->pc_type != 0 && p->pc_type != 2 && p->pc_type != 5)  // d_op_zmobius.C:929-1080
       throw Error{CPSB_ERR_UNSUPPORTED, "zMobius MatInv: ZMOB_PC_SYM2, ORIG and SYM3 only (as the reference)"};
     cudaStream_t st = ctx().stream;
+    CallPool pool(st);
     Operator op(&h->g, *p, P64, 1);
     const long n = op.nsites();
     const Geom &g = op.geom;
@@ -797,6 +816,7 @@ int cpsb_dminus(cpsb_gauge h, const cpsb_dirac_params *p, double *out, const dou
       throw Error{CPSB_ERR_ARG, "Dminus is a Mobius / zMobius operator"};
     if (!out || !in) throw Error{CPSB_ERR_ARG, "null vector"};
     cudaStream_t st = ctx().stream;
+    CallPool pool(st);
     Operator op(&h->g, *p, P64, 1);
     const long n = op.nsites();
     if (out < in + 48 * n && in < out + 48 * n) throw Error{CPSB_ERR_ARG, "out and in overlap"};
@@ -842,6 +862,7 @@ int cpsb_minresext(cpsb_gauge h, const cpsb_dirac_params *p, double *psi, const 
     for (int i = 0; i < degree; i++)
       if (!v[i] || !vm[i]) throw Error{CPSB_ERR_ARG, "null previous solution"};
     cudaStream_t st = ctx().stream;
+    CallPool pool(st);
     Operator op(&h->g, *p, P64, 1);
     const long n = op.nsites();
     const Geom &g = op.geom;

@@ -18,6 +18,8 @@
 #include <string.h>
 
 #include <atomic>
+#include <map>
+#include <mutex>
 
 #include "host.h"
 #include "cg_state.h"
@@ -44,20 +46,137 @@ Context &ctx() {
   return c;
 }
 
-DevBuf::DevBuf(size_t n) { alloc(n); }
-void DevBuf::alloc(size_t n) {
-  if (p) {
-    cudaFree(p);
-    p = nullptr;
-    bytes = 0;
+// ----------------------------------------------------------------- memory
+namespace {
+thread_local bool t_pool_on = false;
+thread_local cudaStream_t t_pool_stream = nullptr;
+std::mutex pool_mu;
+std::map<int, cudaMemPool_t> &pools() {  // one per device, kept until exit
+  static std::map<int, cudaMemPool_t> m;
+  return m;
+}
+// The pool of the current device, made on first use; nullptr where the device
+// has none.
+cudaMemPool_t call_pool() {
+  int dev = 0;
+  CK(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lk(pool_mu);
+  auto it = pools().find(dev);
+  if (it != pools().end()) return it->second;
+  cudaMemPool_t pool = nullptr;
+  int ok = 0;
+  size_t fr = 0, tot = 0;
+  if (cudaDeviceGetAttribute(&ok, cudaDevAttrMemoryPoolsSupported, dev) == cudaSuccess && ok &&
+      cudaMemGetInfo(&fr, &tot) == cudaSuccess) {
+    cudaMemPoolProps props;
+    memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    if (cudaMemPoolCreate(&pool, &props) == cudaSuccess) {
+      unsigned long long keep = tot / 8;
+      if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+        cudaMemPoolDestroy(pool);
+        pool = nullptr;
+      }
+    } else {
+      pool = nullptr;
+    }
   }
+  cudaGetLastError();
+  pools()[dev] = pool;
+  return pool;
+}
+}  // namespace
+
+// A stream under capture allocates as before the pool: the memory of a captured
+// allocation would belong to the graph.
+CallPool::CallPool(cudaStream_t st) : was_on(t_pool_on), was(t_pool_stream) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  t_pool_on = cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
+  if (!t_pool_on) cudaGetLastError();
+  t_pool_stream = st;
+  // The call starts after the work queued on the legacy stream, as when every
+  // reduction slot was cleared there: callers that fill device vectors on the
+  // default stream and pass no stream rely on it.
+  if (t_pool_on) {
+    const cudaError_t e = cudaStreamSynchronize(cudaStreamLegacy);
+    if (e != cudaSuccess) {
+      t_pool_on = was_on;  // no destructor runs for a constructor that throws
+      t_pool_stream = was;
+      CK(e);
+    }
+  }
+}
+CallPool::~CallPool() {
+  t_pool_on = was_on;
+  t_pool_stream = was;
+}
+NoCallPool::NoCallPool() : was_on(t_pool_on) { t_pool_on = false; }
+NoCallPool::~NoCallPool() { t_pool_on = was_on; }
+
+void trim_pool() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  std::lock_guard<std::mutex> lk(pool_mu);
+  auto it = pools().find(dev);
+  if (it != pools().end() && it->second) cudaMemPoolTrimTo(it->second, 0);
+  cudaGetLastError();
+}
+
+DevBuf::DevBuf(size_t n) { alloc(n); }
+void DevBuf::release() {
+  if (!p) return;
+  if (pooled) cudaFreeAsync(p, stream);
+  else cudaFree(p);
+  p = nullptr;
+  bytes = 0;
+}
+void DevBuf::alloc(size_t n) {
+  release();
   if (n == 0) return;
-  CK(cudaMalloc(&p, n));
+  pooled = false;
+  if (t_pool_on) {
+    if (cudaMemPool_t pool = call_pool()) {
+      const cudaError_t e = cudaMallocFromPoolAsync(&p, n, pool, t_pool_stream);
+      if (e == cudaSuccess) {
+        pooled = true;
+        stream = t_pool_stream;
+        bytes = n;
+        return;
+      }
+      p = nullptr;
+      if (e != cudaErrorMemoryAllocation) CK(e);
+      cudaGetLastError();  // no room beside what the pool holds: the plain allocation below
+    }
+  }
+  cudaError_t e = cudaMalloc(&p, n);
+  if (e == cudaErrorMemoryAllocation) {
+    // what the pool keeps, freed once the work behind it is done
+    cudaGetLastError();
+    p = nullptr;
+    cudaDeviceSynchronize();
+    trim_pool();
+    e = cudaMalloc(&p, n);
+  }
+  if (e != cudaSuccess) p = nullptr;
+  CK(e);
   bytes = n;
 }
-DevBuf::~DevBuf() {
-  if (p) cudaFree(p);
+void DevBuf::zero() {
+  if (pooled) {
+    CK(cudaMemsetAsync(p, 0, bytes, stream));
+    return;
+  }
+  // cudaMemset goes to the legacy stream, which does not order against the
+  // library's non-blocking streams, so wait for it here.
+  CK(cudaMemset(p, 0, bytes));
+  CK(cudaStreamSynchronize(cudaStreamLegacy));
 }
+DevBuf::~DevBuf() { release(); }
 
 size_t field_bytes(int prec, long nsites) {
   if (prec == P64) return (size_t)nsites * 192;
@@ -96,11 +215,7 @@ RedSlot::RedSlot() {
   // partials: grid_blocks cap (148*16) * MAX_RHS; + ticket + padding
   const size_t nparts = 148 * 16 * MAX_RHS;
   buf.alloc(nparts * sizeof(double) + 256);
-  // The ticket must be zero before the first kernel that uses the slot runs.
-  // cudaMemset goes to the legacy stream, which does not order against the
-  // library's non-blocking streams, so wait for it here.
-  CK(cudaMemset(buf.p, 0, buf.bytes));
-  CK(cudaStreamSynchronize(cudaStreamLegacy));
+  buf.zero();  // the ticket must be zero before the first kernel that uses the slot runs
 }
 Reduce RedSlot::r(double *result) {
   Reduce q;
@@ -118,6 +233,7 @@ GaugePtr Gauge::ptr(int prec) {
     if (!recon_ok)
       throw Error{CPSB_ERR_UNSUPPORTED,
                   "gauge field is not SU(3) to reduced-precision accuracy; recon-12 storage unavailable"};
+    NoCallPool keep;  // stays with the gauge field
     b.alloc((size_t)n4cb * 2 * 4 * (prec == P32 ? 48 : 24));
     CK(launch_gauge_pack(prec, b.p, (const double *)canon.p, dims, bc_t, ctx().stream));
     CK(cudaStreamSynchronize(ctx().stream));
@@ -329,7 +445,12 @@ static void zmobius_setup(Operator &op, const cpsb_dirac_params &pp) {
   t[0].post_on = t[1].post_on = t[4].post_on = t[9].post_on = t[10].post_on = 1;
   t[2].pre_on = t[2].post_on = 1;
   op.ztab.alloc(sizeof(ZM5Tab) * NT);
-  CK(cudaMemcpy(op.ztab.p, t.data(), sizeof(ZM5Tab) * NT, cudaMemcpyHostToDevice));
+  if (op.ztab.pooled) {
+    CK(cudaMemcpyAsync(op.ztab.p, t.data(), sizeof(ZM5Tab) * NT, cudaMemcpyHostToDevice, op.ztab.stream));
+    CK(cudaStreamSynchronize(op.ztab.stream));  // t leaves scope here
+  } else {
+    CK(cudaMemcpy(op.ztab.p, t.data(), sizeof(ZM5Tab) * NT, cudaMemcpyHostToDevice));
+  }
   op.kappa_b = kb[0].real();
 }
 

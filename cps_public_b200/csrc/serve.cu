@@ -269,6 +269,7 @@ int cpsb_serve_create(cpsb_server *out, int slots, double hbm_fraction, unsigned
     if (!out || slots < 1 || slots > 64) throw Error{CPSB_ERR_ARG, "bad server handle / slot count"};
     if (!(hbm_fraction > 0 && hbm_fraction <= 1) && hbm_bytes == 0)
       throw Error{CPSB_ERR_ARG, "give hbm_fraction in (0, 1] or hbm_bytes > 0"};
+    trim_pool();
     size_t fr = 0, tot = 0;
     CK(cudaMemGetInfo(&fr, &tot));
     size_t budget = hbm_fraction > 0 && hbm_fraction <= 1 ? (size_t)(hbm_fraction * (double)fr) : fr;

@@ -429,8 +429,10 @@ CgSolver *get_solver(Gauge *G, const cpsb_dirac_params &p, int sloppy, int nrhs)
   auto &m = solvers();
   auto it = m.find(k);
   if (it != m.end()) return it->second.get();
-  CgSolver *s = new CgSolver(G, p, sloppy, nrhs);
-  m[k].reset(s);
+  NoCallPool keep;  // a cached solver outlives the call
+  std::unique_ptr<CgSolver> made(new CgSolver(G, p, sloppy, nrhs));
+  CgSolver *s = made.get();
+  m[k] = std::move(made);
   return s;
 }
 
