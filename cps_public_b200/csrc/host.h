@@ -286,11 +286,12 @@ cudaError_t launch_persistent_cg(const DslashArgs &base, double mkappa2, SpinorP
 // cached one, taken under its lock).
 int multishift(Gauge *G, const cpsb_dirac_params &p, const cpsb_cg_arg &a, Field &b64, std::vector<Field> &x,
                const double *shift, int nshift, double *rsd, int type, const double *alpha, cpsb_solve_result *res,
-               cudaStream_t st, CgSolver *refiner = nullptr);
+               cudaStream_t st, CgSolver *refiner = nullptr, bool spare = true);
 // nvec source vectors with the same shifts solved together (multishift.cu):
 // chi and every x[s] hold nvec x n sites; rsd[q * nshift + s]; res[nvec].
 int multishift_multi(Gauge *G, const cpsb_dirac_params &p, const cpsb_cg_arg &a, int nvec, Field &chi,
                      std::vector<Field> &x, const double *shift, int nshift, double *rsd, int type,
-                     const double *alpha, cpsb_solve_result *res, cudaStream_t st, CgSolver *refiner = nullptr);
+                     const double *alpha, cpsb_solve_result *res, cudaStream_t st, CgSolver *refiner = nullptr,
+                     bool spare = true);
 
 }  // namespace cpsb

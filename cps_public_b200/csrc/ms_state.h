@@ -12,6 +12,17 @@ namespace cpsb {
 
 constexpr int MAX_SHIFT = 32;
 
+// Iterations whose updates of the shifts s >= 1 are applied together (see
+// ms_shift_update_kernel).
+constexpr int MS_GROUP = 4;
+
+// What one iteration does to the shifts s >= 1: psi_s -= bs_s p_s for the shifts
+// in x_mask, then p_s = z_s r + as_s p_s for those in p_mask.
+struct MsStep {
+  double bs[MAX_SHIFT], z[MAX_SHIFT], as[MAX_SHIFT];
+  unsigned x_mask, p_mask;            // both 0: the vector did not take part
+};
+
 struct MsState {
   double a, b, bp, c, cp, pp;         // d = d_mm + shift[0]*pp
   double z[2][MAX_SHIFT];
@@ -29,6 +40,7 @@ struct MsState {
   int type;                           // 0 MULTI, 1 SINGLE
   int k;                              // iterations performed (the init step is k = 0)
   int max_iter;
+  MsStep step[MS_GROUP];              // the iterations not yet applied to the shifts s >= 1
   int done;                           // set when every shift converged or k reached max_iter
   int breakdown;
 };

@@ -6,9 +6,11 @@
 // c*z_s^2 < RsdCG_s^2 |chi|^2, and the reported residual is the iterated
 // absolute one, sqrt(c z_s^2).  One iteration is three launch groups --
 // MatPcDagMatPc on p_0 (its fused norm gives |M p_0|^2), the residual update
-// whose last block advances every scalar recurrence, and one pass that updates
-// all solutions and search directions while reading r once -- captured as a
-// CUDA graph and replayed in batches.
+// whose last block advances every scalar recurrence, and the updates of the
+// solutions and search directions -- captured as a CUDA graph and replayed in
+// batches.  The next iteration needs the direction of shift 0 only; the other
+// shifts are brought up to date once per MS_GROUP iterations from the residuals of
+// the group (ms_shift_update_kernel).
 //
 // Several source vectors with the same shifts (the pseudofermions of an RHMC
 // force or action evaluation, alg_action_rational.C:259-359) are solved
@@ -39,76 +41,99 @@ struct ShiftPtrs {
 // The scalar step of one vector after its residual update, with cnew = |r|^2
 // and d = <p_0, (A + shift_0) p_0>: the initial step (minvcg.C:148-196) or
 // iteration k (:224-254, 283-301) with the per-shift convergence checks, then
-// the scalars of the next direction update (:206-222).
-__device__ void ms_advance(MsState *S, double cnew, double d) {
-  const int ns = S->nshift;
+// the scalars of the next direction update (:206-222).  A warp, lane s for shift s:
+// one thread walking the shifts waits for dependent global accesses (12^3x16, Ls 8,
+// FP32, 8 shifts, 2 vectors: the solve 63.6 -> 63.2 ms).
+__device__ __forceinline__ void ms_advance(MsState *S, double cnew, double d, int slot, int s) {
+  static_assert(MAX_SHIFT == 32, "a lane per shift");
+  const int ns = S->nshift, k = S->k;
+  const bool in = s < ns, upper = in && s > 0;
   const double cp = S->c;
-  S->cp = cp;
-  if (!(d != 0.0) || !isfinite(cnew)) {
-    S->breakdown = 1;
-    S->done = 1;
-  } else if (S->k == 0) {
-    const double b0 = -cp / d;
-    S->b = b0;
-    S->z[0][0] = 1.0;
-    S->z[1][0] = 1.0;
-    S->bs[0] = b0;
-    S->iz = 1;
-    for (int s = 1; s < ns; s++) {
-      S->z[0][s] = 1.0;
-      S->z[1][s] = 1.0 / (1.0 - b0 * (S->mass[s] - S->mass[0]));
-      S->bs[s] = b0 * S->z[1][s];
-    }
-    S->c = cnew;
-    for (int s = 0; s < ns; s++) S->conv_prev[s] = 0;
-    if (cnew < S->rsd_sq[0]) S->done = 1;
+  double c = cp, b = S->b, bp = S->bp;
+  int iz = S->iz, done = S->done;
+  const double dm = in ? S->mass[s] - S->mass[0] : 0.0;
+  int conv = in ? S->conv[s] : 1, conv_prev = in ? S->conv_prev[s] : 1;
+  double z0 = in ? S->z[0][s] : 1.0, z1 = in ? S->z[1][s] : 1.0, bs = in ? S->bs[s] : 0.0;
+  const bool broken = !(d != 0.0) || !isfinite(cnew);
+  if (broken) {
+    done = 1;
+  } else if (k == 0) {
+    b = -cp / d;
+    z0 = 1.0;
+    z1 = s == 0 ? 1.0 : 1.0 / (1.0 - b * dm);
+    bs = s == 0 ? b : b * z1;
+    iz = 1;
+    c = cnew;
+    conv_prev = 0;
+    if (cnew < S->rsd_sq[0]) done = 1;
   } else {
     const double a = S->a;
-    S->bp = S->b;
-    const double bp = S->bp;
+    bp = b;
     const double b1 = -cp / d;
-    S->b = b1;
-    S->bs[0] = b1;
-    const int iz = 1 - S->iz;
-    S->iz = iz;
-    for (int s = 1; s < ns; s++) {
-      if (S->conv[s]) continue;
-      const double ztmp = S->z[1 - iz][s] * S->z[iz][s] * bp /
-                          (b1 * a * (S->z[iz][s] - S->z[1 - iz][s]) +
-                           S->z[iz][s] * bp * (1 - b1 * (S->mass[s] - S->mass[0])));
-      S->bs[s] = b1 * ztmp / S->z[1 - iz][s];
-      S->z[iz][s] = ztmp;
+    b = b1;
+    iz = 1 - iz;
+    double zn = iz ? z1 : z0;          // the older value, replaced by the new one
+    const double zc = iz ? z0 : z1;
+    if (s == 0) bs = b1;
+    if (upper && !conv) {
+      const double ztmp = zc * zn * bp / (b1 * a * (zn - zc) + zn * bp * (1 - b1 * dm));
+      bs = b1 * ztmp / zc;
+      zn = ztmp;
     }
-    S->c = cnew;
-    for (int s = 0; s < ns; s++) S->conv_prev[s] = S->conv[s];
-    for (int s = 0; s < ns; s++) {
-      if (S->conv[s]) continue;
-      const double css = cnew * S->z[iz][s] * S->z[iz][s];
+    if (iz) z1 = zn;
+    else z0 = zn;
+    c = cnew;
+    conv_prev = conv;
+    if (in && !conv) {
+      const double css = cnew * zn * zn;
       if (css < S->rsd_sq[s]) {
-        S->conv[s] = 1;
+        conv = 1;
         S->css[s] = css;
-        S->conv_iter[s] = S->k;
+        S->conv_iter[s] = k;
       }
     }
-    int all = S->conv[0];
-    if (all)
-      for (int s = 0; s < ns; s++)
-        if (!S->conv[s]) all = 0;
-    if (all || S->k >= S->max_iter) S->done = 1;
+    if (__all_sync(0xffffffffu, conv) || k >= S->max_iter) done = 1;
   }
-  S->k += 1;
-  const double an = S->c / S->cp;
-  S->a = an;
-  const int iz = S->iz;
-  for (int s = 1; s < ns; s++) S->as[s] = an * (S->z[iz][s] * S->bs[s]) / (S->z[1 - iz][s] * S->b);
+  const double an = c / cp;
+  const double as = an * ((iz ? z1 : z0) * bs) / ((iz ? z0 : z1) * b);
+  MsStep &t = S->step[slot];
+  const unsigned xm = __ballot_sync(0xffffffffu, upper && !conv_prev);
+  const unsigned pm = __ballot_sync(0xffffffffu, upper && !done && !conv);
+  __syncwarp();  // every lane has read the scalars
+  if (in) {
+    S->z[0][s] = z0;
+    S->z[1][s] = z1;
+    S->bs[s] = bs;
+    S->conv[s] = conv;
+    S->conv_prev[s] = conv_prev;
+    if (s > 0) {
+      S->as[s] = as;
+      t.bs[s] = bs;
+      t.z[s] = iz ? z1 : z0;
+      t.as[s] = as;
+    }
+  }
+  if (s == 0) {
+    S->c = c;
+    S->cp = cp;
+    S->b = b;
+    S->bp = bp;
+    S->a = an;
+    S->iz = iz;
+    S->k = k + 1;
+    S->done = done;
+    if (broken) S->breakdown = 1;
+    t.x_mask = xm;
+    t.p_mask = pm;
+  }
 }
 
-// r = r + b (Ap + shift0 p0), b = -c/d; |r|^2; the last block advances the
-// scalars.  Grid row y is vector y (entries [y n, (y+1) n)); the rows of
+// rout = rin + b (Ap + shift0 p0), b = -c/d; |r|^2; the last block advances the
+// scalars and files the iteration under `slot` of its group.  Grid row y is vector y (entries [y n, (y+1) n)); the rows of
 // finished vectors do no work but take part in the reduction's ticket.
 template <int P, int NT>
-__global__ void __launch_bounds__(NT) ms_r_update_kernel(Geom g, SpinorPtr r, SpinorPtr Ap, SpinorPtr p0, MsBatch *B,
-                                                         Reduce red) {
+__global__ void __launch_bounds__(NT) ms_r_update_kernel(Geom g, SpinorPtr rout, SpinorPtr rin, SpinorPtr Ap,
+                                                         SpinorPtr p0, MsBatch *B, int slot, Reduce red) {
   typedef typename PrecTraits<P>::real T;
   __shared__ double sh[NT / 32];
   const int q = blockIdx.y;
@@ -121,7 +146,7 @@ __global__ void __launch_bounds__(NT) ms_r_update_kernel(Geom g, SpinorPtr r, Sp
     const T b = (T)(-S->c / d), tm0 = (T)m0;
     for (long j = (long)blockIdx.x * NT + threadIdx.x; j < n; j += (long)gridDim.x * NT) {
       const long i = q * n + j;
-      Spinor<T> rv = load_spinor<P>(r, i);
+      Spinor<T> rv = load_spinor<P>(rin, i);
       const Spinor<T> av = load_spinor<P>(Ap, i);
       if (m0 != 0.0) {
         const Spinor<T> pv = load_spinor<P>(p0, i);
@@ -135,31 +160,36 @@ __global__ void __launch_bounds__(NT) ms_r_update_kernel(Geom g, SpinorPtr r, Sp
 #pragma unroll
           for (int c = 0; c < 3; c++) rv.c[s][c] = cscale(b, av.c[s][c]) + rv.c[s][c];
       }
-      store_spinor<P>(r, i, rv);
+      store_spinor<P>(rout, i, rv);
       acc += norm2(rounded<P>(rv));
     }
   }
   const double bs = block_sum<NT>(acc, sh);
   if (threadIdx.x == 0) red.partial[q * gridDim.x + blockIdx.x] = bs;
   if (last_block(red.ticket, gridDim.x * gridDim.y)) {
+    __shared__ double cnew[MAX_RHS];
     for (int v = 0; v < (int)gridDim.y; v++) {
-      const double cnew = ordered_sum<NT>(red.partial + v * gridDim.x, gridDim.x, sh);
-      if (threadIdx.x == 0 && !B->done_applied[v]) {
-        MsState *Sv = &B->s[v];
-        ms_advance(Sv, cnew, B->d_mm[v] + Sv->mass[0] * Sv->pp);
-      }
-      __syncthreads();
+      const double t = ordered_sum<NT>(red.partial + v * gridDim.x, gridDim.x, sh);
+      if (threadIdx.x == 0) cnew[v] = t;
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    for (int v = threadIdx.x >> 5; v < (int)gridDim.y; v += NT / 32) {
+      MsState *Sv = &B->s[v];
+      if (!B->done_applied[v]) ms_advance(Sv, cnew[v], B->d_mm[v] + Sv->mass[0] * Sv->pp, slot, lane);
+      else if (lane == 0) Sv->step[slot].x_mask = Sv->step[slot].p_mask = 0;
     }
   }
 }
 
 // psi_s += -bs_s p_s (shifts not frozen at the start of the iteration), then
-// the next directions p_0 = a p_0 + r, p_s = z_s r + as_s p_s; r read once.
-// Grid row y is vector y; its last block sets done_applied after the update
-// of the final iteration.
+// the next directions p_0 = a p_0 + r, p_s = z_s r + as_s p_s; r read once.  Of the
+// shifts below `upto`: 1 where the others follow per group, else all.  Grid row y
+// is vector y; its last block sets done_applied after the update of the final
+// iteration.
 template <int P, int PX, int NT>
 __global__ void __launch_bounds__(NT) ms_xp_update_kernel(Geom g, SpinorPtr r, ShiftPtrs p, ShiftPtrs psi, MsBatch *B,
-                                                          Reduce red) {
+                                                          int upto, Reduce red) {
   typedef typename PrecTraits<P>::real T;
   typedef typename PrecTraits<PX>::real TX;
   __shared__ double sh[NT / 32];
@@ -168,7 +198,7 @@ __global__ void __launch_bounds__(NT) ms_xp_update_kernel(Geom g, SpinorPtr r, S
   const long n = (long)g.n4cb * g.ls;
   double acc = 0;
   if (!B->done_applied[q]) {
-    const int ns = S->nshift;
+    const int ns = min(upto, S->nshift);
     const bool single = S->type == 1;
     const bool done = S->done != 0;
     const int iz = S->iz;
@@ -232,6 +262,107 @@ __global__ void __launch_bounds__(NT) ms_xp_update_kernel(Geom g, SpinorPtr r, S
   }
 }
 
+// The shifts s >= 1 of the `count` iterations filed in step[0..count), with r[j]
+// the residual after iteration j: psi_s -= bs_s p_s, p_s = z_s r + as_s p_s, one
+// iteration after the other, with p_s and psi_s read and written once for the
+// group.  The operations on an element and their order are those of one pass per
+// iteration, so the grouping does not change a result.  Bound by HBM: 4 vectors per
+// running shift and MS_GROUP residuals per group instead of 4 vectors per shift
+// and one residual per iteration.  DWF 16^3x32, Ls 12, 12 shifts, FP64: 442 us an
+// iteration for all shifts before; now 121 us for shift 0 (5 vectors) and 487 us
+// per group for the others, the 250-iteration solve 304 -> 250 ms.
+// Every operation acts on single reals and p, r and psi have the same layout
+// (FP64, or FP32 for both), so a thread takes one 16-byte chunk at a time through
+// all shifts, with few registers and every warp access contiguous.
+// SINGLE: the contributions of an iteration are summed over the shifts first
+// (acc[j]), then added to psi.
+template <int P> struct MsChunk { typedef double2 V; typedef double T; };
+template <> struct MsChunk<P32> { typedef float4 V; typedef float T; };
+__device__ __forceinline__ double2 axpy_chunk(double a, double2 x, double2 y) {
+  return make_double2(a * x.x + y.x, a * x.y + y.y);
+}
+__device__ __forceinline__ float4 axpy_chunk(float a, float4 x, float4 y) {
+  return make_float4(a * x.x + y.x, a * x.y + y.y, a * x.z + y.z, a * x.w + y.w);
+}
+__device__ __forceinline__ double2 lin_chunk(double a, double2 x, double b, double2 y) {
+  return make_double2(a * x.x + b * y.x, a * x.y + b * y.y);
+}
+__device__ __forceinline__ float4 lin_chunk(float a, float4 x, float b, float4 y) {
+  return make_float4(a * x.x + b * y.x, a * x.y + b * y.y, a * x.z + b * y.z, a * x.w + b * y.w);
+}
+
+struct MsGroup {
+  SpinorPtr r[MS_GROUP];
+};
+
+template <int P, int NT>
+__global__ void __launch_bounds__(NT) ms_shift_update_kernel(Geom g, MsGroup R, ShiftPtrs p, ShiftPtrs psi,
+                                                             const MsBatch *B, int count) {
+  typedef typename MsChunk<P>::V V;
+  typedef typename MsChunk<P>::T T;
+  constexpr int NCH = P == P64 ? 12 : 6;
+  __shared__ T f[MAX_SHIFT][MS_GROUP], z[MAX_SHIFT][MS_GROUP], as[MAX_SHIFT][MS_GROUP];
+  __shared__ unsigned xm[MS_GROUP], pm[MS_GROUP];
+  const int q = blockIdx.y;
+  const MsState *S = &B->s[q];
+  const int ns = S->nshift;
+  const bool single = S->type == 1;
+  for (int t = threadIdx.x; t < ns * MS_GROUP; t += NT) {
+    const int s = t / MS_GROUP, j = t % MS_GROUP;
+    const MsStep &st = S->step[j];
+    if (s == 0) {
+      xm[j] = j < count ? st.x_mask : 0u;
+      pm[j] = j < count ? st.p_mask : 0u;
+    } else if (j < count) {
+      f[s][j] = (T)(single ? -st.bs[s] * S->alpha[s] : -st.bs[s]);
+      z[s][j] = (T)st.z[s];
+      as[s][j] = (T)st.as[s];
+    }
+  }
+  __syncthreads();
+  unsigned all_x = 0, all_p = 0;
+#pragma unroll
+  for (int j = 0; j < MS_GROUP; j++) {
+    all_x |= xm[j];
+    all_p |= pm[j];
+  }
+  if (!(all_x | all_p)) return;
+  const V zero = V();
+  const long n = (long)g.n4cb * g.ls * NCH;
+  for (long i = (long)blockIdx.x * NT + threadIdx.x; i < n; i += (long)gridDim.x * NT) {
+    const long c = q * n + i;
+    V rv[MS_GROUP], acc[MS_GROUP];
+#pragma unroll
+    for (int j = 0; j < MS_GROUP; j++) {
+      rv[j] = pm[j] ? ((const V *)R.r[j].data)[c] : zero;
+      acc[j] = zero;
+    }
+    for (int s = 1; s < ns; s++) {
+      const unsigned bit = 1u << s;
+      if (!((all_x | all_p) & bit)) continue;
+      V pv = ((const V *)p.v[s].data)[c];
+      V xv = !single && (all_x & bit) ? ((const V *)psi.v[s].data)[c] : zero;
+#pragma unroll
+      for (int j = 0; j < MS_GROUP; j++) {
+        if (xm[j] & bit) {
+          if (single) acc[j] = axpy_chunk(f[s][j], pv, acc[j]);
+          else xv = axpy_chunk(f[s][j], pv, xv);
+        }
+        if (pm[j] & bit) pv = lin_chunk(z[s][j], rv[j], as[s][j], pv);
+      }
+      if (all_p & bit) ((V *)p.v[s].data)[c] = pv;
+      if (!single && (all_x & bit)) ((V *)psi.v[s].data)[c] = xv;
+    }
+    if (single) {
+      V xv = ((const V *)psi.v[0].data)[c];
+#pragma unroll
+      for (int j = 0; j < MS_GROUP; j++)
+        if (xm[j]) xv = axpy_chunk((T)1, acc[j], xv);
+      ((V *)psi.v[0].data)[c] = xv;
+    }
+  }
+}
+
 static int ms_blocks(long n) {
   long nb = (n + 255) / 256;
   if (nb > 148L * 8) nb = 148L * 8;
@@ -239,21 +370,30 @@ static int ms_blocks(long n) {
 }
 
 // g: the geometry of all vectors (g.nrhs of them, one grid row each).
-cudaError_t launch_ms_r_update(int prec, const Geom &g, SpinorPtr r, SpinorPtr Ap, SpinorPtr p0, MsBatch *B,
-                               Reduce red, cudaStream_t st) {
+cudaError_t launch_ms_r_update(int prec, const Geom &g, SpinorPtr rout, SpinorPtr rin, SpinorPtr Ap, SpinorPtr p0,
+                               MsBatch *B, int slot, Reduce red, cudaStream_t st) {
   const dim3 grid(ms_blocks((long)g.n4cb * g.ls), g.nrhs);
-  if (prec == P64) ms_r_update_kernel<P64, 256><<<grid, 256, 0, st>>>(g, r, Ap, p0, B, red);
-  else if (prec == P32) ms_r_update_kernel<P32, 256><<<grid, 256, 0, st>>>(g, r, Ap, p0, B, red);
-  else ms_r_update_kernel<P16, 256><<<grid, 256, 0, st>>>(g, r, Ap, p0, B, red);
+  if (prec == P64) ms_r_update_kernel<P64, 256><<<grid, 256, 0, st>>>(g, rout, rin, Ap, p0, B, slot, red);
+  else if (prec == P32) ms_r_update_kernel<P32, 256><<<grid, 256, 0, st>>>(g, rout, rin, Ap, p0, B, slot, red);
+  else ms_r_update_kernel<P16, 256><<<grid, 256, 0, st>>>(g, rout, rin, Ap, p0, B, slot, red);
   return launched();
 }
 
 cudaError_t launch_ms_xp_update(int prec, int px, const Geom &g, SpinorPtr r, const ShiftPtrs &p, const ShiftPtrs &psi,
-                                MsBatch *B, Reduce red, cudaStream_t st) {
+                                MsBatch *B, int upto, Reduce red, cudaStream_t st) {
   const dim3 grid(ms_blocks((long)g.n4cb * g.ls), g.nrhs);
-  if (prec == P64 && px == P64) ms_xp_update_kernel<P64, P64, 256><<<grid, 256, 0, st>>>(g, r, p, psi, B, red);
-  else if (prec == P32 && px == P32) ms_xp_update_kernel<P32, P32, 256><<<grid, 256, 0, st>>>(g, r, p, psi, B, red);
-  else if (prec == P16 && px == P32) ms_xp_update_kernel<P16, P32, 256><<<grid, 256, 0, st>>>(g, r, p, psi, B, red);
+  if (prec == P64 && px == P64) ms_xp_update_kernel<P64, P64, 256><<<grid, 256, 0, st>>>(g, r, p, psi, B, upto, red);
+  else if (prec == P32 && px == P32) ms_xp_update_kernel<P32, P32, 256><<<grid, 256, 0, st>>>(g, r, p, psi, B, upto, red);
+  else if (prec == P16 && px == P32) ms_xp_update_kernel<P16, P32, 256><<<grid, 256, 0, st>>>(g, r, p, psi, B, upto, red);
+  else return cudaErrorInvalidValue;
+  return launched();
+}
+
+cudaError_t launch_ms_shift_update(int prec, const Geom &g, const MsGroup &R, const ShiftPtrs &p, const ShiftPtrs &psi,
+                                   const MsBatch *B, int count, cudaStream_t st) {
+  const dim3 grid(ms_blocks((long)g.n4cb * g.ls), g.nrhs);
+  if (prec == P64) ms_shift_update_kernel<P64, 256><<<grid, 256, 0, st>>>(g, R, p, psi, B, count);
+  else if (prec == P32) ms_shift_update_kernel<P32, 256><<<grid, 256, 0, st>>>(g, R, p, psi, B, count);
   else return cudaErrorInvalidValue;
   return launched();
 }
@@ -276,12 +416,13 @@ Scal2 scal_all(double a, double b) {
 // nvec source vectors solved together.  chi: nvec x n FP64 (packed, vector q at
 // entries [q n, (q+1) n)); x: outputs, FP64 fields of nvec x n, nshift of them
 // for MULTI, one for SINGLE; rsd[q * nshift + s]: stop_rsd of shift s for
-// vector q on entry, its reported residual on return; res[q]: the report of
-// vector q (iters: CPS's iteration count of its Krylov phase plus, with
+// vector q on entry, its reported residual on return; spare: MS_GROUP - 1 Krylov
+// vectors per source beyond the ones of the recurrence may be used if they fit;
+// res[q]: the report of vector q (iters: CPS's iteration count of its Krylov phase plus, with
 // refinement, the refinement iterations).
 int multishift_multi(Gauge *G, const cpsb_dirac_params &p, const cpsb_cg_arg &a, int nvec, Field &chi,
                      std::vector<Field> &x, const double *shift, int nshift, double *rsd, int type,
-                     const double *alpha, cpsb_solve_result *res, cudaStream_t st, CgSolver *refiner) {
+                     const double *alpha, cpsb_solve_result *res, cudaStream_t st, CgSolver *refiner, bool spare) {
   auto t0 = std::chrono::steady_clock::now();
   if (nshift < 1 || nshift > MAX_SHIFT) throw Error{CPSB_ERR_ARG, "nshift must be in [1, 32]"};
   if (nvec < 1 || nvec > MAX_RHS) throw Error{CPSB_ERR_ARG, "nvec must be in [1, 16]"};
@@ -296,7 +437,7 @@ int multishift_multi(Gauge *G, const cpsb_dirac_params &p, const cpsb_cg_arg &a,
   const long n = g.nsites;       // all vectors
   const long n1 = n / nvec;      // one vector
   const int px = prec == P64 ? P64 : P32;
-  Field r(prec, n), Ap(prec, n);
+  Field Ap(prec, n);
   std::vector<Field> pv(nshift);
   const int nx = ktype == 1 ? 1 : nshift;
   std::vector<Field> psi(nx);
@@ -307,6 +448,24 @@ int multishift_multi(Gauge *G, const cpsb_dirac_params &p, const cpsb_cg_arg &a,
   }
   RedSlot red_d, red_r, red_p, red_m;
   DevBuf dres(sizeof(double) * MAX_RHS);
+  const int batch = a.batch > 0 ? a.batch : (graph_loops_enabled() ? 4 : 16);
+  // The shifts s >= 1 are updated once per `group` iterations, which keeps the
+  // residuals of the group: with `spare` and room for the vectors, else the group is
+  // one iteration and the residual is updated in place.  SINGLE takes groups of one:
+  // shift 0 and the others add to the same vector, so a longer group would change
+  // the order of the sum.  16-bit Krylov vectors, whose rounding is per entry and
+  // iteration, keep one pass over all shifts per iteration.
+  const bool grouped = prec != P16 && nshift > 1;
+  int group = grouped && spare && ktype == 0 ? (batch < MS_GROUP ? batch : MS_GROUP) : 1;
+  std::vector<std::unique_ptr<Field>> rf;
+  try {
+    for (int j = 0; j < group; j++) rf.emplace_back(new Field(prec, n));
+  } catch (const Error &e) {
+    if (e.code != CPSB_ERR_OOM || rf.empty()) throw;
+    rf.resize(1);
+    group = 1;
+  }
+  Field &r = *rf[(batch - 1) % group];  // where a batch's first iteration reads the residual
   // |chi_q|^2 (FmatEvlMInv's NormSqGlbSum, f_dwf_base.C:248)
   double chi_norm[MAX_RHS];
   CK(launch_redot(P64, g, chi.ptr(), chi.ptr(), red_m.r((double *)dres.p), st));
@@ -365,12 +524,17 @@ int multishift_multi(Gauge *G, const cpsb_dirac_params &p, const cpsb_cg_arg &a,
     const int *skip = B->done_applied;
     op.mdagm(Ap, pv[0], &rd, skip, st);  // uncaptured application: tunes the launch shapes
     CK(cudaMemcpyAsync(state.p, &init, sizeof(MsBatch), cudaMemcpyHostToDevice, st));
-    const int batch = a.batch > 0 ? a.batch : (graph_loops_enabled() ? 4 : 16);
+    MsGroup rg;
+    memset(&rg, 0, sizeof(rg));
+    for (int j = 0; j < group; j++) rg.r[j] = rf[j]->ptr();
     auto record = [&]() {
       for (int j = 0; j < batch; j++) {
+        const int slot = j % group, prev = (j == 0 ? batch - 1 : j - 1) % group;
         op.mdagm(Ap, pv[0], &rd, skip, st);
-        CK(launch_ms_r_update(prec, g, r.ptr(), Ap.ptr(), pv[0].ptr(), B, rr, st));
-        CK(launch_ms_xp_update(prec, px, g, r.ptr(), pp_, xx_, B, rp, st));
+        CK(launch_ms_r_update(prec, g, rg.r[slot], rg.r[prev], Ap.ptr(), pv[0].ptr(), B, slot, rr, st));
+        CK(launch_ms_xp_update(prec, px, g, rg.r[slot], pp_, xx_, B, grouped ? 1 : nshift, rp, st));
+        if (grouped && (slot == group - 1 || j == batch - 1))
+          CK(launch_ms_shift_update(prec, g, rg, pp_, xx_, B, slot + 1, st));
       }
     };
     // one graph launch runs batches on the device until every vector is done
@@ -504,8 +668,8 @@ int multishift_multi(Gauge *G, const cpsb_dirac_params &p, const cpsb_cg_arg &a,
 
 int multishift(Gauge *G, const cpsb_dirac_params &p, const cpsb_cg_arg &a, Field &chi, std::vector<Field> &x,
                const double *shift, int nshift, double *rsd, int type, const double *alpha, cpsb_solve_result *res,
-               cudaStream_t st, CgSolver *refiner) {
-  return multishift_multi(G, p, a, 1, chi, x, shift, nshift, rsd, type, alpha, res, st, refiner);
+               cudaStream_t st, CgSolver *refiner, bool spare) {
+  return multishift_multi(G, p, a, 1, chi, x, shift, nshift, rsd, type, alpha, res, st, refiner, spare);
 }
 
 }  // namespace cpsb

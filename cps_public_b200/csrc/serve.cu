@@ -161,7 +161,8 @@ void Server::run_item(const ServeItem &it, cudaStream_t st) {
     std::unique_ptr<CgSolver> refiner;
     if (r.a.precision != P64) refiner.reset(new CgSolver(G, r.p, r.a.precision, 1));
     const int rc = multishift(G, r.p, r.a, chi, xs, r.shift.data(), nshift, r.rsd, r.ms_type,
-                              r.alpha.empty() ? nullptr : r.alpha.data(), r.res.data(), st, refiner.get());
+                              r.alpha.empty() ? nullptr : r.alpha.data(), r.res.data(), st, refiner.get(),
+                              false);  // no vectors beyond the item's footprint
     for (int i = 0; i < nvec; i++) {
       CK(launch_unpack(P64, (double *)stage.p, xs[i].ptr(), g1, st));
       CK(cudaMemcpyAsync(r.x[i], stage.p, each, cudaMemcpyDeviceToHost, st));

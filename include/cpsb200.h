@@ -256,7 +256,8 @@ int cpsb_minvcg_dev(cpsb_gauge h, const cpsb_dirac_params *p, const cpsb_cg_arg 
  * CPSB_SINGLE): the solutions.  rsd[q * nshift + s]: stop_rsd of shift s for
  * vector q on entry, its reported residual on return.  res[q]: the report of
  * vector q.  nvec <= 16.  Device memory: (nshift + 3) Krylov vectors and nsol
- * solutions per source vector, plus the FP64 inputs and outputs. */
+ * solutions per source vector, plus the FP64 inputs and outputs; three Krylov
+ * vectors more per source where they fit. */
 int cpsb_minvcg_multi(cpsb_gauge h, const cpsb_dirac_params *p, const cpsb_cg_arg *a, int nvec, double **x,
                       const double *const *b, const double *shift, int nshift, double *rsd, int type,
                       const double *alpha, cpsb_solve_result *res);
