@@ -576,8 +576,6 @@ cudaError_t launch_persistent_cg(const DslashArgs &base, double mkappa2, SpinorP
   memset(&P, 0, sizeof(P));
   for (int k = 0; k < 4; k++) {
     P.ph[k] = base;
-    P.ph[k].rg = 1;
-    P.ph[k].rgroup = g.nrhs;
     P.ph[k].torder = 0;
     P.ph[k].skip = nullptr;
     memset(&P.ph[k].red, 0, sizeof(Reduce));

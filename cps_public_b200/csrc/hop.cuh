@@ -12,11 +12,9 @@
 // Work decomposition (the column layout of cpsb_device.cuh).  A field is a
 // set of columns, one per (4-D checkerboard site x, slice class k), each
 // holding the class's slices of that site as consecutive entries.  A work unit
-// is a tile of TX consecutive columns of one class, taken for a group of RG
-// right-hand sides at a time (RG = 1 or all of them; A.rg); a block sweeps its
-// unit's columns x slices x right-hand sides of the group.  Thread t owns
-// slice t % C (C the column height), right-hand side (t / C) % RG and column
-// t / (C RG), so:
+// is a tile of TX consecutive columns of one class; a block sweeps its unit's
+// columns x slices x right-hand sides.  Thread t owns slice t % C (C the column
+// height) of column t / C for every right-hand side, so:
 //  * the 32 lanes of a warp read whole neighbour columns per 16-byte chunk --
 //    contiguous 128-byte segments that start on 128-byte boundaries when C is
 //    a multiple of 8 (DWF Ls 16: 4 columns x 8 slices per warp);
@@ -28,8 +26,7 @@
 //    of the packed FP32x2 instructions (launch shapes without the table, LC
 //    false, read recon-12 links from global memory per thread instead);
 //  * neighbour column offsets are computed once per unit;
-//  * units run in tile order, optionally inside groups of A.rgroup right-hand
-//    sides (the group slowest), and the grid holds only the blocks resident at
+//  * units run in tile order, and the grid holds only the blocks resident at
 //    once, so the columns that blocks in flight touch -- their own and their
 //    neighbours' up to one time slice away -- are read while they sit in L2.
 //
@@ -321,107 +318,116 @@ template <int MU, bool POS> __device__ __forceinline__ HfX2 iproject(const Raw<P
   return h;
 }
 
-// U h (DAG = false) or U^dag h (DAG = true) for both spins; the link elements
-// come from shared memory as (ur, ur, ui, ui), row-major.
-template <bool DAG> __device__ __forceinline__ HfX2 umul_x2(const float4 *l, const HfX2 &h) {
-  HfX2 o;
-  float2 nh[3];
-#pragma unroll
-  for (int k = 0; k < 3; k++) nh[k] = DAG ? f2(-h.re[k].x, -h.re[k].y) : f2(-h.im[k].x, -h.im[k].y);
-#pragma unroll
-  for (int r = 0; r < 3; r++) {
-    float2 re = f2b(0.f), im = f2b(0.f);
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      const float4 e = l[DAG ? 3 * k + r : 3 * r + k];
-      const float2 ur = lo2(e), ui = hi2(e);
-      re = fma2(ur, h.re[k], re);
-      im = fma2(ur, h.im[k], im);
-      if (DAG) {  // conj(u) h: re += ui Im h, im -= ui Re h
-        re = fma2(ui, h.im[k], re);
-        im = fma2(ui, nh[k], im);
-      } else {    // u h: re -= ui Im h, im += ui Re h
-        re = fma2(ui, nh[k], re);
-        im = fma2(ui, h.re[k], im);
-      }
-    }
-    o.re[r] = re;
-    o.im[r] = im;
+// A link as the operand pairs of the packed arithmetic: element i (row-major) as
+// (ur, ur), (ui, ui), from the unit's shared-memory table or from registers
+// (launch shapes without the table).
+struct LinkTab {
+  const float4 *l;
+  __device__ __forceinline__ float4 operator[](int i) const { return l[i]; }
+};
+struct LinkReg {
+  Link<float> u;
+  __device__ __forceinline__ float4 operator[](int i) const {
+    const cplx<float> e = u.u[i / 3][i % 3];
+    return make_float4(e.re, e.re, e.im, e.im);
   }
-  return o;
+};
+
+// A reconstructible link (rows 0 and 1) as loaded.
+template <int P> struct RawLink;
+template <> struct RawLink<P32> { float4 v[3]; };
+template <> struct RawLink<P16> { uint2 v[3]; };
+template <int P> __device__ __forceinline__ RawLink<P> load_raw_link(const GaugePtr &g, int par, int mu, int x) {
+  RawLink<P> r;
+  auto *b = (decltype(&r.v[0]))const_cast<void *>(g.data) + (long)((par * 4 + mu) * 3) * g.n4cb + x;
+#pragma unroll
+  for (int k = 0; k < 3; k++) r.v[k] = __ldg(b + k * g.n4cb);
+  return r;
+}
+__device__ __forceinline__ Link<float> unpack_link(const RawLink<P32> &r) {
+  Link<float> l;
+  l.u[0][0] = mk(r.v[0].x, r.v[0].y); l.u[0][1] = mk(r.v[0].z, r.v[0].w);
+  l.u[0][2] = mk(r.v[1].x, r.v[1].y); l.u[1][0] = mk(r.v[1].z, r.v[1].w);
+  l.u[1][1] = mk(r.v[2].x, r.v[2].y); l.u[1][2] = mk(r.v[2].z, r.v[2].w);
+  reconstruct_row2(l);
+  return l;
+}
+__device__ __forceinline__ Link<float> unpack_link(const RawLink<P16> &r) {
+  const float q = 1.0f / 32767.0f;
+  Link<float> l;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const int e0 = 2 * k, e1 = 2 * k + 1;
+    l.u[e0 / 3][e0 % 3] = mk(dec16(r.v[k].x, 0) * q, dec16(r.v[k].x, 1) * q);
+    l.u[e1 / 3][e1 % 3] = mk(dec16(r.v[k].y, 0) * q, dec16(r.v[k].y, 1) * q);
+  }
+  reconstruct_row2(l);
+  return l;
 }
 
-// The same with the link in registers (launch shapes without the link table).
-template <bool DAG> __device__ __forceinline__ HfX2 umul_x2r(const Link<float> &u, const HfX2 &h) {
-  HfX2 o;
-  float2 nh[3];
-#pragma unroll
-  for (int k = 0; k < 3; k++) nh[k] = DAG ? f2(-h.re[k].x, -h.re[k].y) : f2(-h.im[k].x, -h.im[k].y);
-#pragma unroll
-  for (int r = 0; r < 3; r++) {
-    float2 re = f2b(0.f), im = f2b(0.f);
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      const cplx<float> e = DAG ? u.u[k][r] : u.u[r][k];
-      const float2 ur = f2b(e.re), ui = f2b(e.im);
-      re = fma2(ur, h.re[k], re);
-      im = fma2(ur, h.im[k], im);
-      if (DAG) {
-        re = fma2(ui, h.im[k], re);
-        im = fma2(ui, nh[k], im);
-      } else {
-        re = fma2(ui, nh[k], re);
-        im = fma2(ui, h.re[k], im);
-      }
-    }
-    o.re[r] = re;
-    o.im[r] = im;
-  }
-  return o;
-}
-
-// Accumulator: the upper pair (spins 0,1), and the lower pair split into the
-// terms that arrive in natural lane order (ln: spins 2,3) and swapped (ls:
-// spins 3,2), merged once at the end.
-struct AccX2 { float2 ure[3], uim[3], lnre[3], lnim[3], lsre[3], lsim[3]; };
+// Accumulator: the upper pair (spins 0, 1) and the lower pair, whose lanes hold
+// spins (3, 2) while the x and y neighbours are added (their terms arrive
+// swapped) and spins (2, 3) from the z neighbours on (swap_lower between).
+struct AccX2 { float2 ure[3], uim[3], lre[3], lim[3]; };
 
 __device__ __forceinline__ void zero_x2(AccX2 &a) {
 #pragma unroll
-  for (int c = 0; c < 3; c++) a.ure[c] = a.uim[c] = a.lnre[c] = a.lnim[c] = a.lsre[c] = a.lsim[c] = f2b(0.f);
+  for (int c = 0; c < 3; c++) a.ure[c] = a.uim[c] = a.lre[c] = a.lim[c] = f2b(0.f);
 }
-
-// acc += f * (full spinor rebuilt from the multiplied half spinor h): the
-// reconstruction of accum_reconstruct() in cpsb_device.cuh.
-template <int MU> __device__ __forceinline__ void accum_x2(AccX2 &a, const HfX2 &h, float sg, float f) {
-  const float s = f * sg;
+__device__ __forceinline__ void swap_lower(AccX2 &a) {
 #pragma unroll
   for (int c = 0; c < 3; c++) {
-    a.ure[c] = fma2(f2b(f), h.re[c], a.ure[c]);
-    a.uim[c] = fma2(f2b(f), h.im[c], a.uim[c]);
-    if (MU == 0) {         // psi2 += -i sg h1, psi3 += -i sg h0
-      a.lsre[c] = fma2(f2b(s), h.im[c], a.lsre[c]);
-      a.lsim[c] = fma2(f2b(-s), h.re[c], a.lsim[c]);
-    } else if (MU == 1) {  // psi2 += sg h1, psi3 -= sg h0
-      a.lsre[c] = fma2(f2(-s, s), h.re[c], a.lsre[c]);
-      a.lsim[c] = fma2(f2(-s, s), h.im[c], a.lsim[c]);
+    a.lre[c] = swp(a.lre[c]);
+    a.lim[c] = swp(a.lim[c]);
+  }
+}
+
+// acc += f * (full spinor rebuilt from U h, or U^dag h for DAGL): the link multiply
+// and the reconstruction of accum_reconstruct() in cpsb_device.cuh, row by row.
+template <int MU, bool DAGL, class LK>
+__device__ __forceinline__ void mul_accum_x2(AccX2 &a, const LK &l, const HfX2 &h, float sg, float f) {
+  const float s = f * sg;
+#pragma unroll
+  for (int r = 0; r < 3; r++) {
+    float2 re, im;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const float4 e = l[DAGL ? 3 * k + r : 3 * r + k];
+      const float2 ur = lo2(e), ui = hi2(e);
+      const float2 hr = h.re[k], hi = h.im[k];
+      re = k == 0 ? mul2(ur, hr) : fma2(ur, hr, re);
+      im = k == 0 ? mul2(ur, hi) : fma2(ur, hi, im);
+      // U: re -= ui Im h, im += ui Re h; U^dag: re += ui Im h, im -= ui Re h
+      const float2 nh = DAGL ? f2(-hr.x, -hr.y) : f2(-hi.x, -hi.y);
+      re = fma2(ui, DAGL ? hi : nh, re);
+      im = fma2(ui, DAGL ? nh : hr, im);
+    }
+    a.ure[r] = fma2(f2b(f), re, a.ure[r]);
+    a.uim[r] = fma2(f2b(f), im, a.uim[r]);
+    if (MU == 0) {         // psi2 += -i sg h1, psi3 += -i sg h0 (lanes swapped)
+      a.lre[r] = fma2(f2b(s), im, a.lre[r]);
+      a.lim[r] = fma2(f2b(-s), re, a.lim[r]);
+    } else if (MU == 1) {  // psi2 += sg h1, psi3 -= sg h0 (lanes swapped)
+      a.lre[r] = fma2(f2(-s, s), re, a.lre[r]);
+      a.lim[r] = fma2(f2(-s, s), im, a.lim[r]);
     } else if (MU == 2) {  // psi2 += -i sg h0, psi3 += i sg h1
-      a.lnre[c] = fma2(f2(s, -s), h.im[c], a.lnre[c]);
-      a.lnim[c] = fma2(f2(-s, s), h.re[c], a.lnim[c]);
+      a.lre[r] = fma2(f2(s, -s), im, a.lre[r]);
+      a.lim[r] = fma2(f2(-s, s), re, a.lim[r]);
     } else {               // psi2 += sg h0, psi3 += sg h1
-      a.lnre[c] = fma2(f2b(s), h.re[c], a.lnre[c]);
-      a.lnim[c] = fma2(f2b(s), h.im[c], a.lnim[c]);
+      a.lre[r] = fma2(f2b(s), re, a.lre[r]);
+      a.lim[r] = fma2(f2b(s), im, a.lim[r]);
     }
   }
 }
 
-__device__ __forceinline__ SpX2 merge_x2(const AccX2 &a) {
+__device__ __forceinline__ SpX2 spinor_x2(const AccX2 &a) {
   SpX2 o;
 #pragma unroll
   for (int c = 0; c < 3; c++) {
     o.re[0][c] = a.ure[c];
     o.im[0][c] = a.uim[c];
-    o.re[1][c] = add2(a.lnre[c], swp(a.lsre[c]));
-    o.im[1][c] = add2(a.lnim[c], swp(a.lsim[c]));
+    o.re[1][c] = a.lre[c];
+    o.im[1][c] = a.lim[c];
   }
   return o;
 }
@@ -613,48 +619,81 @@ __device__ __forceinline__ Spinor<double> hop_entry_64(const DslashArgs &A, cons
   return acc;
 }
 
-// The same for FP32 / 16-bit storage in packed FP32x2 arithmetic.
-template <int P, bool LC, bool DAG, int DEPTH>
-__device__ __forceinline__ SpX2 hop_entry_x2(const DslashArgs &A, const HopCtx &hc, unsigned rb) {
+// The neighbours of the packed hop in the order +x -x +y -y +z -z +t -t (see AccX2):
+// the m-th one's index in HopCtx.
+__device__ __forceinline__ constexpr int nb_order(int m) { return (m >> 1) + 4 * (m & 1); }
+
+// The neighbour loads in flight ahead of the arithmetic of the packed hop: the
+// next one, and at DEPTH 2 the one after it.
+template <int P> struct Ahead { Raw<P> n1, n2; };
+template <int P, int DEPTH>
+__device__ __forceinline__ void start_ahead(Ahead<P> &q, const DslashArgs &A, const HopCtx &hc, unsigned rb) {
+  q.n1 = load_raw<P>(A.in, rb + (unsigned)hc.nb[nb_order(0)]);
+  if (DEPTH >= 2) q.n2 = load_raw<P>(A.in, rb + (unsigned)hc.nb[nb_order(1)]);
+}
+
+// The same for FP32 / 16-bit storage in packed FP32x2 arithmetic.  On entry q holds
+// the first neighbours; CROSS: when `more`, it leaves holding those of the entry
+// at rbn (the thread's next right-hand side), so that their latency passes during the
+// last neighbours and the epilogue.
+template <int P, bool LC, bool DAG, int DEPTH, bool CROSS>
+__device__ __forceinline__ SpX2 hop_entry_x2(const DslashArgs &A, const HopCtx &hc, unsigned rb, Ahead<P> &q,
+                                             unsigned rbn, bool more) {
   constexpr float sdag = DAG ? -1.f : 1.f;
-  const void *lk = hc.lk;
   const int par_out = hc.par_out, x = hc.x;
-  const float4 *l32 = (const float4 *)lk;
+  const float4 *l32 = (const float4 *)hc.lk;
   AccX2 acc;
   zero_x2(acc);
-  // DEPTH (1 or 2): neighbours whose loads are in flight ahead of the one computed
-  Raw<P> nxt, nx2;
-  nxt = load_raw<P>(A.in, rb + (unsigned)hc.nb[0]);
-  if (DEPTH >= 2) nx2 = load_raw<P>(A.in, rb + (unsigned)hc.nb[1]);
+  RawLink<P> nl;  // !LC: the next neighbour's link, loaded one neighbour ahead
+  if (!LC) nl = load_raw_link<P>(A.U, par_out, 0, x);
 #pragma unroll
-  for (int j = 0; j < 8; j++) {
-    const Raw<P> cur = nxt;
-    if (DEPTH >= 2) {
-      nxt = nx2;
-      if (j < 6) nx2 = load_raw<P>(A.in, rb + (unsigned)hc.nb[j + 2]);
-    } else if (j < 7) {
-      nxt = load_raw<P>(A.in, rb + (unsigned)hc.nb[j + 1]);
+  for (int m = 0; m < 8; m++) {
+    const int j = nb_order(m);  // neighbour: mu = m / 2, forward then backward
+    if (m == 4) swap_lower(acc);
+    const Raw<P> cur = q.n1;
+    const int ahead = m + DEPTH;
+    if (ahead < 8) {
+      const Raw<P> v = load_raw<P>(A.in, rb + (unsigned)hc.nb[nb_order(ahead & 7)]);
+      if (DEPTH >= 2) q.n1 = q.n2, q.n2 = v;
+      else q.n1 = v;
+    } else {
+      if (DEPTH >= 2) q.n1 = q.n2;
+      if (CROSS && more) {
+        const Raw<P> v = load_raw<P>(A.in, rbn + (unsigned)hc.nb[nb_order(ahead & 7)]);
+        if (DEPTH >= 2) q.n2 = v;
+        else q.n1 = v;
+      }
     }
     float nrm;
     const float sg = j < 4 ? -sdag : sdag;
-    // FP32: unpack, then project; 16-bit: project on the integers (iproject)
-    SpX2 v;
-    if constexpr (P == P32) v = unpack(cur, &nrm);
-    else nrm = cur.nrm;
-    const float4 *lj = l32 + j * 9;
-    Link<float> lr;
+    LinkTab lt;
+    LinkReg lr;
+    lt.l = l32 + j * 9;
     if (!LC) {
-      lr = j < 4 ? load_link<P>(A.U, par_out, j & 3, x) : load_link<P>(A.U, 1 - par_out, j & 3, hc.xn[j]);
-      if ((j == 3 && hc.flip_f) || (j == 7 && hc.flip_b)) nrm = -nrm;
+      lr.u = unpack_link(nl);
+      if (m < 7) {
+        const int jn = nb_order(m + 1);
+        nl = jn < 4 ? load_raw_link<P>(A.U, par_out, jn & 3, x) : load_raw_link<P>(A.U, 1 - par_out, jn & 3, hc.xn[jn]);
+      }
     }
-#define CPSB_NB(MU)                                                                            \
-  {                                                                                            \
-    HfX2 h;                                                                                    \
-    if constexpr (P == P16) h = sg > 0.f ? iproject<MU, true>(cur) : iproject<MU, false>(cur); \
-    else h = project_x2<MU>(v, sg);                                                            \
-    const HfX2 uh = LC ? (j < 4 ? umul_x2<false>(lj, h) : umul_x2<true>(lj, h))                \
-                       : (j < 4 ? umul_x2r<false>(lr, h) : umul_x2r<true>(lr, h));             \
-    accum_x2<MU>(acc, uh, sg, nrm);                                                            \
+#define CPSB_NB(MU)                                                                          \
+  {                                                                                          \
+    HfX2 h;                                                                                  \
+    /* FP32: unpack, then project; 16-bit: project on the integers (iproject) */             \
+    if constexpr (P == P16) {                                                                \
+      nrm = cur.nrm;                                                                         \
+      h = sg > 0.f ? iproject<MU, true>(cur) : iproject<MU, false>(cur);                     \
+    } else {                                                                                 \
+      h = project_x2<MU>(unpack(cur, &nrm), sg);                                             \
+    }                                                                                        \
+    if (!LC && ((j == 3 && hc.flip_f) || (j == 7 && hc.flip_b))) nrm = -nrm;                 \
+    if constexpr (LC) {                                                                      \
+      if (j < 4) mul_accum_x2<MU, false>(acc, lt, h, sg, nrm);                               \
+      else mul_accum_x2<MU, true>(acc, lt, h, sg, nrm);                                      \
+    } else {                                                                                 \
+      if (j < 4) mul_accum_x2<MU, false>(acc, lr, h, sg, nrm);                               \
+      else mul_accum_x2<MU, true>(acc, lr, h, sg, nrm);                                      \
+    }                                                                                        \
   }
     switch (j & 3) {
       case 0: CPSB_NB(0) break;
@@ -677,17 +716,24 @@ __device__ __forceinline__ SpX2 hop_entry_x2(const DslashArgs &A, const HopCtx &
       if (!DAG) {
         acc.ure[c] = fma2(cm, vm.re[c], acc.ure[c]);
         acc.uim[c] = fma2(cm, vm.im[c], acc.uim[c]);
-        acc.lnre[c] = fma2(cp, vp.re[c], acc.lnre[c]);
-        acc.lnim[c] = fma2(cp, vp.im[c], acc.lnim[c]);
+        acc.lre[c] = fma2(cp, vp.re[c], acc.lre[c]);
+        acc.lim[c] = fma2(cp, vp.im[c], acc.lim[c]);
       } else {
-        acc.lnre[c] = fma2(cm, vm.re[c], acc.lnre[c]);
-        acc.lnim[c] = fma2(cm, vm.im[c], acc.lnim[c]);
+        acc.lre[c] = fma2(cm, vm.re[c], acc.lre[c]);
+        acc.lim[c] = fma2(cm, vm.im[c], acc.lim[c]);
         acc.ure[c] = fma2(cp, vp.re[c], acc.ure[c]);
         acc.uim[c] = fma2(cp, vp.im[c], acc.uim[c]);
       }
     }
   }
-  return merge_x2(acc);
+  return spinor_x2(acc);
+}
+
+template <int P, bool LC, bool DAG, int DEPTH>
+__device__ __forceinline__ SpX2 hop_entry_x2(const DslashArgs &A, const HopCtx &hc, unsigned rb) {
+  Ahead<P> q;
+  start_ahead<P, DEPTH>(q, A, hc, rb);
+  return hop_entry_x2<P, LC, DAG, DEPTH, false>(A, hc, rb, q, 0u, false);
 }
 
 // The context of slice sp of tile column xl (checkerboard site x, class k)
@@ -718,19 +764,33 @@ __device__ __forceinline__ void entry_ctx(HopCtx &hc, const DslashArgs &A, const
   hc.lk = dsh + L.links + (size_t)xl * LSTR * 16;
 }
 
+// An entry's lines to L2.
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+template <int P> __device__ __forceinline__ void prefetch_entry(const SpinorPtr &f, unsigned i) {
+  constexpr int NCH = P == P64 ? 12 : P == P32 ? 6 : 3;
+  const char *b = entry_ptr<NCH, const char>(f.data, i);
+#pragma unroll
+  for (int k = 0; k < NCH; k++) prefetch_l2(b + 128 * k);
+  if (P == P16) prefetch_l2(f.norm + i);
+}
+
 // LC: links from the unit's shared-memory table (otherwise each entry loads
 // and reconstructs its own, which suits columns of one or two entries).
 //
-// Thread t of a block owns slice sp = t % C0 of column xl = t / (C0*RG) and
-// the right-hand sides rl, rl + RG, ... with rl = (t / C0) % RG (A.rg, set by
-// the launcher so that C0*RG lanes divide a warp: with DWF Ls 16 and 12
-// right-hand sides a warp is one column x 8 slices x 4 right-hand sides, and
-// every link read is a broadcast).  The grid holds no more blocks than are
-// resident at once, so the units in flight are one contiguous run of tiles and
-// their neighbour columns are read while they are in L2.
+// Thread t of a block owns slice sp = t % C0 of column xl = t / C0 for every
+// right-hand side.  The grid holds no more blocks than are resident at once, so
+// the units in flight are one contiguous run of tiles and their neighbour columns
+// are read while they are in L2.
+// FP32 / 16-bit: the lower accumulators serve the swapped terms of the x and y
+// neighbours first and the natural ones of z and t after one lane swap, 12 registers
+// less than a set for each (FP32 16^3x32, Ls 16, 12 right-hand sides: 778 -> 743 us, 1:
+// 91 -> 83 us; 16-bit x12 713 -> 707).  Tried on the same shapes and slower: two and
+// three right-hand sides a thread sharing each link read, or four in a warp on one
+// column, although the link table's reads are 47% of the 16-bit kernel's L1
+// wavefronts (x12: 777, 1068 and 799 us).
 // CGR: 0 none, 1 the fused residual update r -= alpha A p, 2 the same for the
 // shifted operator, r -= alpha (A p + shift p).
-template <int P, int NT, int MINB, bool LC, bool XPAY, bool NORM, int CGR, bool DAG, int DEPTH>
+template <int P, int NT, int MINB, bool LC, bool XPAY, bool NORM, int CGR, bool DAG, int DEPTH, bool CROSS>
 __global__ void __launch_bounds__(NT, MINB) hop_kernel(DslashArgs A) {
   const Geom &g = A.g;
   extern __shared__ __align__(16) unsigned char dsh[];
@@ -743,25 +803,19 @@ __global__ void __launch_bounds__(NT, MINB) hop_kernel(DslashArgs A) {
     cg_alpha[threadIdx.x] = S->rr[threadIdx.x] / (S->d[threadIdx.x] + S->shift * S->pp[threadIdx.x]);
   }
   const int C0 = g.cs[0];
-  const int RG = A.rg;
-  const int TX = NT / (C0 * RG);
+  const int TX = NT / C0;
   const HopShm L = hop_shm(TX, NT, g.nrhs, NORM || CGR, LC);
   double *nrm_sh = (double *)(dsh + L.norm);
   if (NORM || CGR)
     for (int q = 0; q < g.nrhs; q++) nrm_sh[q * NT + threadIdx.x] = 0;
   const int sp = threadIdx.x % C0;                 // slice index of the thread within its column
-  const int rl = (threadIdx.x / C0) % RG;          // right-hand side within the group
-  const int xl = threadIdx.x / (C0 * RG);          // column of the tile
+  const int xl = threadIdx.x / C0;                 // column of the tile
   const int ntiles = (g.n4cb + TX - 1) / TX;
   const int ncls = g.ncls;
-  // units: (group of A.rgroup right-hand sides, tile, class), the group slowest
-  const int G = A.rgroup;
-  const int per_group = ntiles * ncls;
-  const int nunits = per_group * ((g.nrhs + G - 1) / G);
+  const int nunits = ntiles * ncls;
   const unsigned per = (unsigned)g.n4cb * (unsigned)g.ls;
   for (int unit = blockIdx.x; unit < nunits; unit += gridDim.x) {
-    const int grp = unit / per_group, rem = unit - grp * per_group;
-    const int k = rem % ncls, tile = tile_order(g, rem / ncls, TX, A.torder);
+    const int k = unit % ncls, tile = tile_order(g, unit / ncls, TX, A.torder);
     const int par_out = A.five_d ? ((1 - A.cb + k) & 1) : 1 - A.cb;
     __syncthreads();  // the previous unit is done with the tables
     load_unit<P, LC>(A, tile, k, par_out, TX, NT, dsh);
@@ -772,12 +826,15 @@ __global__ void __launch_bounds__(NT, MINB) hop_kernel(DslashArgs A) {
     HopCtx hc;
     entry_ctx<P, LC>(hc, A, dsh, L, xl, x, k, sp, par_out);
     const unsigned own = (k ? (unsigned)g.kb1 : 0u) + (unsigned)x * (unsigned)C + (unsigned)sp;
-    const int rhs_end = min(g.nrhs, (grp + 1) * G);
-    for (int rhs = grp * G + rl; rhs < rhs_end; rhs += RG) {
+    unsigned todo_rhs = 0;  // right-hand sides still iterating
+    if (P != P64)
+      for (int rhs = 0; rhs < g.nrhs; rhs++)
+        if (!(A.skip && A.skip[rhs])) todo_rhs |= 1u << rhs;
+    if constexpr (P == P64) {
+    for (int rhs = 0; rhs < g.nrhs; rhs++) {
       if (A.skip && A.skip[rhs]) continue;
       const unsigned rb = (unsigned)rhs * per;
       const unsigned i = rb + own;
-      if constexpr (P == P64) {
         // ------------------------------------------------ FP64
         Spinor<double> acc = hop_entry_64<P, LC, DAG, DEPTH>(A, hc, rb);
         const double a = A.a;
@@ -796,25 +853,21 @@ __global__ void __launch_bounds__(NT, MINB) hop_kernel(DslashArgs A) {
         if (CGR) {
           const double alpha = cg_alpha[rhs];
           Spinor<double> rv = unpack64(load_raw<P64>(A.cg_r, i));
-          if (CGR == 2 || A.cg_x.data) {
-            const Spinor<double> pv = unpack64(load_raw<P64>(A.cg_p, i));
-            if (CGR == 2) {
-              const double sigma = A.cg->shift;
+          const Spinor<double> pv = unpack64(load_raw<P64>(A.cg_p, i));
+          if (CGR == 2) {
+            const double sigma = A.cg->shift;
 #pragma unroll
-              for (int s2 = 0; s2 < 4; s2++)
+            for (int s2 = 0; s2 < 4; s2++)
 #pragma unroll
-                for (int r = 0; r < 3; r++) acc.c[s2][r] = acc.c[s2][r] + cscale(sigma, pv.c[s2][r]);
-            }
-            if (A.cg_x.data) {
-              // x += alpha p (the solution half of cg_xp_update, blas.cu)
-              Spinor<double> xv = unpack64(load_raw<P64>(A.cg_x, i));
-#pragma unroll
-              for (int s2 = 0; s2 < 4; s2++)
-#pragma unroll
-                for (int r = 0; r < 3; r++) xv.c[s2][r] = cscale(alpha, pv.c[s2][r]) + xv.c[s2][r];
-              store_spinor<P64>(A.cg_x, i, xv);
-            }
+              for (int r = 0; r < 3; r++) acc.c[s2][r] = acc.c[s2][r] + cscale(sigma, pv.c[s2][r]);
           }
+          // x += alpha p (the solution half of cg_xp_update, blas.cu)
+          Spinor<double> xv = unpack64(load_raw<P64>(A.cg_x, i));
+#pragma unroll
+          for (int s2 = 0; s2 < 4; s2++)
+#pragma unroll
+            for (int r = 0; r < 3; r++) xv.c[s2][r] = cscale(alpha, pv.c[s2][r]) + xv.c[s2][r];
+          store_spinor<P64>(A.cg_x, i, xv);
 #pragma unroll
           for (int s2 = 0; s2 < 4; s2++)
 #pragma unroll
@@ -825,9 +878,31 @@ __global__ void __launch_bounds__(NT, MINB) hop_kernel(DslashArgs A) {
           store_spinor<P64>(A.out, i, acc);
           if (NORM) nrm_sh[rhs * NT + threadIdx.x] += norm2(acc);
         }
-      } else {
-        // ------------------------------------------------ FP32 / 16-bit, packed
-        SpX2 o = hop_entry_x2<P, LC, DAG, DEPTH>(A, hc, rb);
+    }
+    } else {
+    // ------------------------------------------------ FP32 / 16-bit, packed
+    unsigned todo = todo_rhs;
+    Ahead<P> q;
+    if (CROSS && todo) start_ahead<P, DEPTH>(q, A, hc, (unsigned)(__ffs(todo) - 1) * per);
+    while (todo) {
+      const int rhs = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const unsigned rb = (unsigned)rhs * per;
+      const unsigned i = rb + own;
+      const unsigned rbn = todo ? (unsigned)(__ffs(todo) - 1) * per : rb;
+      if (!CROSS) start_ahead<P, DEPTH>(q, A, hc, rb);
+      if (P == P16 && CGR) {
+        // The update's operands, 240 bytes an entry, come from L2 when the hop is done:
+        // 1445 -> 1369 us (16^3x32, Ls 16, 12 right-hand sides).  For the xpay operand
+        // alone (863 -> 872 us) and for FP32 (102 -> 114 us on 12^3x24, Ls 10, 3
+        // right-hand sides) the extra instructions cost more.
+        prefetch_entry<P>(A.x, i);
+        prefetch_entry<P>(A.cg_r, i);
+        prefetch_entry<P>(A.cg_p, i);
+        prefetch_entry<P32>(A.cg_x, i);
+      }
+      SpX2 o = hop_entry_x2<P, LC, DAG, DEPTH, CROSS>(A, hc, rb, q, rbn, todo != 0);
+      {
         const float2 a2 = f2b((float)A.a);
         if (XPAY) {
           float xn;
@@ -854,29 +929,24 @@ __global__ void __launch_bounds__(NT, MINB) hop_kernel(DslashArgs A) {
             }
         }
         if (CGR) {
-          // r -= alpha (A p + shift p), A p = o in registers (cg_r_update of blas.cu)
+          // r -= alpha (A p + shift p), A p = o in registers (cg_r_update of blas.cu);
+          // every operand's load before the first store
           const float alpha = (float)cg_alpha[rhs];
-          float rn;
+          float rn, pn, xn;
           SpX2 rv = unpack(load_raw<P>(A.cg_r, i), &rn);
-          float pn = 0.f;
-          SpX2 pv;
-          double sigma = 0.0;
-          if (CGR == 2 || A.cg_x.data) pv = unpack(load_raw<P>(A.cg_p, i), &pn);
-          if (CGR == 2) sigma = A.cg->shift;
-          if (A.cg_x.data) {
-            // x += alpha p in FP32 (the solution half of cg_xp_update, blas.cu)
-            float xn;
-            SpX2 xv = unpack(load_raw<P32>(A.cg_x, i), &xn);
-            const float2 ap = f2b(alpha * pn);
+          const SpX2 pv = unpack(load_raw<P>(A.cg_p, i), &pn);
+          SpX2 xv = unpack(load_raw<P32>(A.cg_x, i), &xn);
+          const double sigma = CGR == 2 ? A.cg->shift : 0.0;
+          // x += alpha p in FP32 (the solution half of cg_xp_update, blas.cu)
+          const float2 ap = f2b(alpha * pn);
 #pragma unroll
-            for (int p = 0; p < 2; p++)
+          for (int p = 0; p < 2; p++)
 #pragma unroll
-              for (int cc = 0; cc < 3; cc++) {
-                xv.re[p][cc] = fma2(ap, pv.re[p][cc], xv.re[p][cc]);
-                xv.im[p][cc] = fma2(ap, pv.im[p][cc], xv.im[p][cc]);
-              }
-            store_x2<P32>(A.cg_x, i, xv);
-          }
+            for (int cc = 0; cc < 3; cc++) {
+              xv.re[p][cc] = fma2(ap, pv.re[p][cc], xv.re[p][cc]);
+              xv.im[p][cc] = fma2(ap, pv.im[p][cc], xv.im[p][cc]);
+            }
+          store_x2<P32>(A.cg_x, i, xv);
           const float2 ma = f2b(-alpha), rs = f2b(rn), ps = f2b((float)sigma * pn);
 #pragma unroll
           for (int p = 0; p < 2; p++)
@@ -897,6 +967,7 @@ __global__ void __launch_bounds__(NT, MINB) hop_kernel(DslashArgs A) {
         }
       }
     }
+    }
   }
   if (NORM || CGR) {
     for (int q = 0; q < g.nrhs; q++) {
@@ -904,17 +975,22 @@ __global__ void __launch_bounds__(NT, MINB) hop_kernel(DslashArgs A) {
       if (threadIdx.x == 0) A.red.partial[q * gridDim.x + blockIdx.x] = bs;
     }
     if (last_block(A.red.ticket, gridDim.x)) {
+      __shared__ double total[MAX_RHS];
       for (int q = 0; q < g.nrhs; q++) {
         const double t = ordered_sum<NT>(A.red.partial + q * gridDim.x, gridDim.x, red);
-        if (threadIdx.x == 0 && !(A.skip && A.skip[q])) {
-          if (!CGR) {
-            A.red.result[q] = t;
-          } else {
-            cg_advance(A.cg, q, t);
-            if (A.red.result) A.red.result[q] = t;
-          }
+        if (threadIdx.x == 0) total[q] = t;
+      }
+      __syncthreads();
+      // the scalar steps of all right-hand sides side by side: each is a chain of
+      // global accesses of about 2 us
+      const int q = threadIdx.x;
+      if (q < g.nrhs && !(A.skip && A.skip[q])) {
+        if (!CGR) {
+          A.red.result[q] = total[q];
+        } else {
+          cg_advance(A.cg, q, total[q]);
+          if (A.red.result) A.red.result[q] = total[q];
         }
-        __syncthreads();
       }
     }
   }
@@ -1097,17 +1173,22 @@ __global__ void __launch_bounds__(NT) hop8_kernel(DslashArgs A) {
       if (threadIdx.x == 0) A.red.partial[q * gridDim.x + blockIdx.x] = bs;
     }
     if (last_block(A.red.ticket, gridDim.x)) {
+      __shared__ double total[MAX_RHS];
       for (int q = 0; q < g.nrhs; q++) {
         const double t = ordered_sum<NT>(A.red.partial + q * gridDim.x, gridDim.x, red);
-        if (threadIdx.x == 0 && !(A.skip && A.skip[q])) {
-          if (!CGR) {
-            A.red.result[q] = t;
-          } else {
-            cg_advance(A.cg, q, t);
-            if (A.red.result) A.red.result[q] = t;
-          }
+        if (threadIdx.x == 0) total[q] = t;
+      }
+      __syncthreads();
+      // the scalar steps of all right-hand sides side by side: each is a chain of
+      // global accesses of about 2 us
+      const int q = threadIdx.x;
+      if (q < g.nrhs && !(A.skip && A.skip[q])) {
+        if (!CGR) {
+          A.red.result[q] = total[q];
+        } else {
+          cg_advance(A.cg, q, total[q]);
+          if (A.red.result) A.red.result[q] = total[q];
         }
-        __syncthreads();
       }
     }
   }
@@ -1143,30 +1224,22 @@ static int resident_blocks(const void *fn, int nt, size_t shm) {
 }
 
 // One launch shape: NT threads, at least MINB resident blocks per SM, link
-// table (LC), right-hand-side grouping (GRP: as many right-hand sides per warp
-// as divide it, else one).  The fused residual update (A.cg) needs the xpay
-// form.
-template <int P, int NT, int MINB, bool LC, bool GRP, int DEPTH>
-static cudaError_t hop_launch_v(DslashArgs A, int xpay, int norm, cudaStream_t st, int rgroup, int torder) {
+// table (LC), neighbours loaded ahead (DEPTH, and CROSS: into the next right-hand
+// side).  The fused residual update (A.cg) needs the xpay form and the solution
+// (A.cg_x).
+template <int P, int NT, int MINB, bool LC, int DEPTH, bool CROSS = false>
+static cudaError_t hop_launch_v(DslashArgs A, int xpay, int norm, cudaStream_t st, int torder) {
   const int C0 = A.g.cs[0];
   if (C0 < 1 || C0 > NT) return cudaErrorNotSupported;
-  int rg = 1;
-  if (GRP)
-    while (rg * 2 <= A.g.nrhs && C0 * rg * 2 <= 32 && 32 % (C0 * rg * 2) == 0) rg *= 2;
-  if (GRP && rg == 1) return cudaErrorNotSupported;  // the same as the ungrouped shape
-  A.rg = rg;
+  if (CROSS && A.g.nrhs == 1) return cudaErrorNotSupported;  // the same as without
   A.torder = torder;
-  // right-hand sides per unit: all, or groups of rgroup (a multiple of rg), so
-  // that the blocks resident at one time touch only a few right-hand sides
-  A.rgroup = rgroup > 0 ? std::max(rg, rgroup / rg * rg) : A.g.nrhs;
-  if (rgroup > 0 && A.rgroup >= A.g.nrhs) return cudaErrorNotSupported;  // the same as all
-  const int TX = NT / (C0 * rg);
+  const int TX = NT / C0;
   if (TX < 1 || (LC && TX > 32)) return cudaErrorNotSupported;  // link tables of more than 32 columns: use !LC
   const bool cgr = A.cg != nullptr;
-  if (cgr && !xpay) return cudaErrorInvalidValue;
+  if (cgr && (!xpay || !A.cg_x.data)) return cudaErrorInvalidValue;
   const HopShm L = hop_shm(TX, NT, A.g.nrhs, norm || cgr, LC);
   if (L.total > 200 * 1024) return cudaErrorNotSupported;
-  const long units = (long)((A.g.n4cb + TX - 1) / TX) * A.g.ncls * ((A.g.nrhs + A.rgroup - 1) / A.rgroup);
+  const long units = (long)((A.g.n4cb + TX - 1) / TX) * A.g.ncls;
   // the opt-in above the 48 KB default is set once per instantiation
   auto opt_in = [&](const void *f, bool &done) -> cudaError_t {
     if (done || L.total + 1024 <= 48 * 1024) return cudaSuccess;
@@ -1177,12 +1250,12 @@ static cudaError_t hop_launch_v(DslashArgs A, int xpay, int norm, cudaStream_t s
   cudaError_t e = cudaSuccess;
 #define CPSB_HOP(XP, NR, CG, D)                                                            \
   {                                                                                        \
-    const void *fn = (const void *)hop_kernel<P, NT, MINB, LC, XP, NR, CG, D, DEPTH>;             \
+    const void *fn = (const void *)hop_kernel<P, NT, MINB, LC, XP, NR, CG, D, DEPTH, CROSS>;             \
     static bool done = false;                                                              \
     e = opt_in(fn, done);                                                                  \
     if (e != cudaSuccess) return e;                                                        \
     const long nb = std::min(units, (long)resident_blocks(fn, NT, L.total));                \
-    hop_kernel<P, NT, MINB, LC, XP, NR, CG, D, DEPTH><<<(unsigned)nb, NT, L.total, st>>>(A);      \
+    hop_kernel<P, NT, MINB, LC, XP, NR, CG, D, DEPTH, CROSS><<<(unsigned)nb, NT, L.total, st>>>(A);      \
   }
 #define CPSB_HOP_D(XP, NR, CG)          \
   if (A.dag) CPSB_HOP(XP, NR, CG, true) \
@@ -1203,7 +1276,7 @@ static cudaError_t hop_launch_v(DslashArgs A, int xpay, int norm, cudaStream_t s
 template <int NT>
 static cudaError_t hop8_launch(const DslashArgs &A, int xpay, int norm, cudaStream_t st) {
   const bool cgr = A.cg != nullptr;
-  if (cgr && !xpay) return cudaErrorInvalidValue;
+  if (cgr && (!xpay || !A.cg_x.data)) return cudaErrorInvalidValue;
   const size_t shm = (size_t)12 * NT * sizeof(double2) + ((norm || cgr) ? (size_t)NT * A.g.nrhs * sizeof(double) : 0);
   const long entries = (long)A.g.n4cb * A.g.ls;  // of one right-hand side
   const long want = (entries + NT / 8 - 1) / (NT / 8);
@@ -1227,27 +1300,33 @@ static cudaError_t hop8_launch(const DslashArgs &A, int xpay, int norm, cudaStre
   return launched();
 }
 
-// Launch shapes the autotuner chooses from: (threads, min blocks per SM, link
-// table, right-hand-side grouping).  Shapes with link tables need columns of at
-// least NT/32 entries (DWF, Mobius); shape 4 serves short columns (Wilson).
+// Launch shapes the autotuner chooses from.  Shapes with link tables need columns of
+// at least NT/32 entries (DWF, Mobius); the ones without serve short columns.
 template <int P>
 static cudaError_t hop_launch_p(const DslashArgs &A, int xpay, int norm, int variant, cudaStream_t st) {
   switch (variant) {
-    // (threads, blocks per SM, link table, RHS per warp lane group, prefetch
-    // depth; RHS per unit, t-fastest tile order).  FP64 keeps fewer blocks
-    // (more registers) and one neighbour less in flight.
-    case 0: return hop_launch_v<P, 128, P == P64 ? 2 : 4, true, false, P == P64 ? 1 : 2>(A, xpay, norm, st, 0, 0);
-    case 1: return hop_launch_v<P, 128, P == P64 ? 3 : 5, true, false, P == P64 ? 1 : 2>(A, xpay, norm, st, 0, 0);
-    case 2: return hop_launch_v<P, 256, P == P64 ? 1 : 2, true, false, P == P64 ? 1 : 2>(A, xpay, norm, st, 0, 0);
-    case 3: return hop_launch_v<P, 256, P == P64 ? 1 : 2, true, false, P == P64 ? 1 : 2>(A, xpay, norm, st, 0, 1);
-    case 4: return hop_launch_v<P, 128, P == P64 ? 2 : 4, false, false, P == P64 ? 1 : 2>(A, xpay, norm, st, 0, 0);
-    case 5: return hop_launch_v<P, 128, P == P64 ? 3 : 5, true, false, P == P64 ? 0 : 1>(A, xpay, norm, st, 0, 0);
-    case 6: return hop_launch_v<P, 128, P == P64 ? 4 : 6, true, false, P == P64 ? 0 : 1>(A, xpay, norm, st, 0, 0);
-    case 7: return hop_launch_v<P, 256, P == P64 ? 1 : 2, true, true, P == P64 ? 1 : 2>(A, xpay, norm, st, 4, 0);
+    // (threads, blocks per SM, link table, neighbours ahead; t-fastest tile
+    // order).  FP64 keeps fewer blocks (more registers) and one neighbour less in
+    // flight.
+    case 0: return hop_launch_v<P, 128, P == P64 ? 2 : 4, true, P == P64 ? 1 : 2>(A, xpay, norm, st, 0);
+    case 1: return hop_launch_v<P, 128, P == P64 ? 3 : 5, true, P == P64 ? 1 : 2>(A, xpay, norm, st, 0);
+    case 2: return hop_launch_v<P, 256, P == P64 ? 1 : 2, true, P == P64 ? 1 : 2>(A, xpay, norm, st, 0);
+    case 3: return hop_launch_v<P, 256, P == P64 ? 1 : 2, true, P == P64 ? 1 : 2>(A, xpay, norm, st, 1);
+    case 4: return hop_launch_v<P, 128, P == P64 ? 2 : 4, false, P == P64 ? 1 : 2>(A, xpay, norm, st, 0);
+    case 5: return hop_launch_v<P, 128, P == P64 ? 3 : 5, true, P == P64 ? 0 : 1>(A, xpay, norm, st, 0);
+    case 6: return hop_launch_v<P, 128, P == P64 ? 4 : 6, true, P == P64 ? 0 : 1>(A, xpay, norm, st, 0);
+    // 16-bit, several right-hand sides: one neighbour ahead, across right-hand sides
+    // (16^3x32, Ls 16, x12: 699 us against 708 for shape 2; Ls 12 without the 5th
+    // direction, x4: 179 against 187).  FP32 entries do not leave the registers.
+    case 7:
+      if constexpr (P == P16) return hop_launch_v<P, 256, 2, true, 1, true>(A, xpay, norm, st, 0);
+      else return cudaErrorNotSupported;
+    // FP32 and 16-bit without the table: one neighbour and its link ahead (Wilson
+    // 24^3x64, FP32: 70 us against 75 for shape 4)
     // FP64: eight lanes per entry, one neighbour each (small lattices)
     case 8:
       if constexpr (P == P64) return hop8_launch<128>(A, xpay, norm, st);
-      else return cudaErrorNotSupported;
+      else return hop_launch_v<P, 128, 4, false, 1>(A, xpay, norm, st, 0);
     default: return cudaErrorNotSupported;
   }
 }

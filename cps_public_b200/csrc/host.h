@@ -188,15 +188,15 @@ struct Operator {
   }
   // MatPcDagMatPc p with the CG residual update fused into its last hop
   // (Wilson / DWF, every precision): |MatPc p|^2 -> red_d, then
-  // r -= alpha (A p + shift p), |r|^2 and the recurrence scalars in S, and with
-  // x given x += alpha p; A p is not stored (scratch receives it only while a
+  // r -= alpha (A p + shift p), |r|^2 and the recurrence scalars in S, and
+  // x += alpha p; A p is not stored (scratch receives it only while a
   // launch shape is being tuned).
   bool can_fuse_cg_r() const { return p.action == CPSB_WILSON || p.action == CPSB_DWF; }
   bool mobius_like() const { return p.action == CPSB_MOBIUS || p.action == CPSB_ZMOBIUS; }
   void matpc_zmobius(const SpinorPtr &out, const SpinorPtr &in, int dag, const Reduce *red, const int *skip,
                      cudaStream_t st);
   void mdagm_cg_r(const SpinorPtr &scratch, const SpinorPtr &in, const Reduce *red_d, const int *skip, CgState *S,
-                  const SpinorPtr &r, const Reduce *red_r, bool shifted, const SpinorPtr *x, cudaStream_t st);
+                  const SpinorPtr &r, const Reduce *red_r, bool shifted, const SpinorPtr &x, cudaStream_t st);
   // Mobius pieces of DiracOpMobius::MatInv (SYM2): out = M5^-1 in
   // (zmobius_m5inv, dag 0); out = D4(cb) in (zmobius_dslash_4, dag 0);
   // out = x + f H5 in (zmobius_kappa_dslash_5_plus_cmplx with factor f, dag 0).

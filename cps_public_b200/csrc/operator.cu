@@ -817,7 +817,7 @@ void Operator::mobius_hop5_add(const SpinorPtr &out, const SpinorPtr &in, const 
 }
 
 void Operator::mdagm_cg_r(const SpinorPtr &scratch, const SpinorPtr &in, const Reduce *red_d, const int *skip,
-                          CgState *S, const SpinorPtr &r, const Reduce *red_r, bool shifted, const SpinorPtr *x,
+                          CgState *S, const SpinorPtr &r, const Reduce *red_r, bool shifted, const SpinorPtr &x,
                           cudaStream_t st) {
   if (!can_fuse_cg_r()) throw Error{CPSB_ERR_UNSUPPORTED, "fused residual update needs the Wilson or DWF operator"};
   matpc(t2.ptr(), in, 0, red_d, skip, st);  // |MatPc p|^2 -> d
@@ -846,7 +846,7 @@ void Operator::mdagm_cg_r(const SpinorPtr &scratch, const SpinorPtr &in, const R
   A.cg_r = r;
   A.cg_p = in;
   A.cg_shift = shifted ? 1 : 0;
-  if (x) A.cg_x = *x;
+  A.cg_x = x;
   CK(launch_dslash(prec, A, 1, 1, v, st));
 }
 

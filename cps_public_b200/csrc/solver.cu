@@ -96,8 +96,7 @@ void CgSolver::launch_batch(int k, cudaStream_t st) {
     if (fused) {
       // the residual update rides on the last hop of MatPcDagMatPc (A p stays in registers)
       // and so does x += alpha p: the x/p kernel then updates p alone
-      const SpinorPtr xp = xx.ptr();
-      op.mdagm_cg_r(ApS.ptr(), pS.ptr(), &rd, S->halt, S, rS.ptr(), &rr, shift != 0.0, &xp, st);
+      op.mdagm_cg_r(ApS.ptr(), pS.ptr(), &rd, S->halt, S, rS.ptr(), &rr, shift != 0.0, xx.ptr(), st);
     } else {
       op.mdagm(ApS, pS, &rd, S->halt, st);
       CK(launch_cg_r_update(op.prec, op.geom, rS.ptr(), ApS.ptr(), pS.ptr(), S, rr, st));
