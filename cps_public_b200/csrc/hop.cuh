@@ -764,6 +764,98 @@ __device__ __forceinline__ void entry_ctx(HopCtx &hc, const DslashArgs &A, const
   hc.lk = dsh + L.links + (size_t)xl * LSTR * 16;
 }
 
+// The CG update of one entry, A p = acc in registers: r -= alpha (A p + shift p) and
+// x += alpha p; returns |r|^2 of the entry (CGR 2: the shift is nonzero).
+template <int CGR>
+__device__ __forceinline__ double cg_epilogue_64(const DslashArgs &A, unsigned i, double alpha, Spinor<double> &acc) {
+  Spinor<double> rv = unpack64(load_raw<P64>(A.cg_r, i));
+  const Spinor<double> pv = unpack64(load_raw<P64>(A.cg_p, i));
+  if (CGR == 2) {
+    const double sigma = A.cg->shift;
+#pragma unroll
+    for (int s2 = 0; s2 < 4; s2++)
+#pragma unroll
+      for (int r = 0; r < 3; r++) acc.c[s2][r] = acc.c[s2][r] + cscale(sigma, pv.c[s2][r]);
+  }
+  // x += alpha p (the solution half of cg_xp_update, blas.cu)
+  Spinor<double> xv = unpack64(load_raw<P64>(A.cg_x, i));
+#pragma unroll
+  for (int s2 = 0; s2 < 4; s2++)
+#pragma unroll
+    for (int r = 0; r < 3; r++) xv.c[s2][r] = cscale(alpha, pv.c[s2][r]) + xv.c[s2][r];
+  store_spinor<P64>(A.cg_x, i, xv);
+#pragma unroll
+  for (int s2 = 0; s2 < 4; s2++)
+#pragma unroll
+    for (int r = 0; r < 3; r++) rv.c[s2][r] = rv.c[s2][r] - cscale(alpha, acc.c[s2][r]);
+  store_spinor<P64>(A.cg_r, i, rv);
+  return norm2(rv);
+}
+template <int P, int CGR>
+__device__ __forceinline__ double cg_epilogue_x2(const DslashArgs &A, unsigned i, float alpha, SpX2 &o) {
+  // r -= alpha (A p + shift p), A p = o in registers (cg_r_update of blas.cu);
+  // every operand's load before the first store
+  float rn, pn, xn;
+  SpX2 rv = unpack(load_raw<P>(A.cg_r, i), &rn);
+  const SpX2 pv = unpack(load_raw<P>(A.cg_p, i), &pn);
+  SpX2 xv = unpack(load_raw<P32>(A.cg_x, i), &xn);
+  const double sigma = CGR == 2 ? A.cg->shift : 0.0;
+  // x += alpha p in FP32 (the solution half of cg_xp_update, blas.cu)
+  const float2 ap = f2b(alpha * pn);
+#pragma unroll
+  for (int p = 0; p < 2; p++)
+#pragma unroll
+    for (int cc = 0; cc < 3; cc++) {
+      xv.re[p][cc] = fma2(ap, pv.re[p][cc], xv.re[p][cc]);
+      xv.im[p][cc] = fma2(ap, pv.im[p][cc], xv.im[p][cc]);
+    }
+  store_x2<P32>(A.cg_x, i, xv);
+  const float2 ma = f2b(-alpha), rs = f2b(rn), ps = f2b((float)sigma * pn);
+#pragma unroll
+  for (int p = 0; p < 2; p++)
+#pragma unroll
+    for (int cc = 0; cc < 3; cc++) {
+      float2 are = o.re[p][cc], aim = o.im[p][cc];
+      if (CGR == 2) {
+        are = fma2(ps, pv.re[p][cc], are);
+        aim = fma2(ps, pv.im[p][cc], aim);
+      }
+      rv.re[p][cc] = fma2(ma, are, P == P16 ? mul2(rv.re[p][cc], rs) : rv.re[p][cc]);
+      rv.im[p][cc] = fma2(ma, aim, P == P16 ? mul2(rv.im[p][cc], rs) : rv.im[p][cc]);
+    }
+  return store_x2<P>(A.cg_r, i, rv);
+}
+
+// The reduction that ends a hop: nrm_sh[q * NT + thread] summed per right-hand side;
+// the last block stores |out|^2 or advances the CG scalars (CGR).
+template <int NT, int CGR>
+__device__ __forceinline__ void hop_reduce(const DslashArgs &A, const double *nrm_sh, double *red) {
+  const Geom &g = A.g;
+  for (int q = 0; q < g.nrhs; q++) {
+    const double bs = block_sum<NT>(nrm_sh[q * NT + threadIdx.x], red);
+    if (threadIdx.x == 0) A.red.partial[q * gridDim.x + blockIdx.x] = bs;
+  }
+  if (last_block(A.red.ticket, gridDim.x)) {
+    __shared__ double total[MAX_RHS];
+    for (int q = 0; q < g.nrhs; q++) {
+      const double t = ordered_sum<NT>(A.red.partial + q * gridDim.x, gridDim.x, red);
+      if (threadIdx.x == 0) total[q] = t;
+    }
+    __syncthreads();
+    // the scalar steps of all right-hand sides side by side: each is a chain of
+    // global accesses of about 2 us
+    const int q = threadIdx.x;
+    if (q < g.nrhs && !(A.skip && A.skip[q])) {
+      if (!CGR) {
+        A.red.result[q] = total[q];
+      } else {
+        cg_advance(A.cg, q, total[q]);
+        if (A.red.result) A.red.result[q] = total[q];
+      }
+    }
+  }
+}
+
 // An entry's lines to L2.
 __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 template <int P> __device__ __forceinline__ void prefetch_entry(const SpinorPtr &f, unsigned i) {
@@ -851,29 +943,7 @@ __global__ void __launch_bounds__(NT, MINB) hop_kernel(DslashArgs A) {
             for (int r = 0; r < 3; r++) acc.c[s2][r] = cscale(a, acc.c[s2][r]);
         }
         if (CGR) {
-          const double alpha = cg_alpha[rhs];
-          Spinor<double> rv = unpack64(load_raw<P64>(A.cg_r, i));
-          const Spinor<double> pv = unpack64(load_raw<P64>(A.cg_p, i));
-          if (CGR == 2) {
-            const double sigma = A.cg->shift;
-#pragma unroll
-            for (int s2 = 0; s2 < 4; s2++)
-#pragma unroll
-              for (int r = 0; r < 3; r++) acc.c[s2][r] = acc.c[s2][r] + cscale(sigma, pv.c[s2][r]);
-          }
-          // x += alpha p (the solution half of cg_xp_update, blas.cu)
-          Spinor<double> xv = unpack64(load_raw<P64>(A.cg_x, i));
-#pragma unroll
-          for (int s2 = 0; s2 < 4; s2++)
-#pragma unroll
-            for (int r = 0; r < 3; r++) xv.c[s2][r] = cscale(alpha, pv.c[s2][r]) + xv.c[s2][r];
-          store_spinor<P64>(A.cg_x, i, xv);
-#pragma unroll
-          for (int s2 = 0; s2 < 4; s2++)
-#pragma unroll
-            for (int r = 0; r < 3; r++) rv.c[s2][r] = rv.c[s2][r] - cscale(alpha, acc.c[s2][r]);
-          store_spinor<P64>(A.cg_r, i, rv);
-          nrm_sh[rhs * NT + threadIdx.x] += norm2(rv);
+          nrm_sh[rhs * NT + threadIdx.x] += cg_epilogue_64<CGR>(A, i, cg_alpha[rhs], acc);
         } else {
           store_spinor<P64>(A.out, i, acc);
           if (NORM) nrm_sh[rhs * NT + threadIdx.x] += norm2(acc);
@@ -929,38 +999,7 @@ __global__ void __launch_bounds__(NT, MINB) hop_kernel(DslashArgs A) {
             }
         }
         if (CGR) {
-          // r -= alpha (A p + shift p), A p = o in registers (cg_r_update of blas.cu);
-          // every operand's load before the first store
-          const float alpha = (float)cg_alpha[rhs];
-          float rn, pn, xn;
-          SpX2 rv = unpack(load_raw<P>(A.cg_r, i), &rn);
-          const SpX2 pv = unpack(load_raw<P>(A.cg_p, i), &pn);
-          SpX2 xv = unpack(load_raw<P32>(A.cg_x, i), &xn);
-          const double sigma = CGR == 2 ? A.cg->shift : 0.0;
-          // x += alpha p in FP32 (the solution half of cg_xp_update, blas.cu)
-          const float2 ap = f2b(alpha * pn);
-#pragma unroll
-          for (int p = 0; p < 2; p++)
-#pragma unroll
-            for (int cc = 0; cc < 3; cc++) {
-              xv.re[p][cc] = fma2(ap, pv.re[p][cc], xv.re[p][cc]);
-              xv.im[p][cc] = fma2(ap, pv.im[p][cc], xv.im[p][cc]);
-            }
-          store_x2<P32>(A.cg_x, i, xv);
-          const float2 ma = f2b(-alpha), rs = f2b(rn), ps = f2b((float)sigma * pn);
-#pragma unroll
-          for (int p = 0; p < 2; p++)
-#pragma unroll
-            for (int cc = 0; cc < 3; cc++) {
-              float2 are = o.re[p][cc], aim = o.im[p][cc];
-              if (CGR == 2) {
-                are = fma2(ps, pv.re[p][cc], are);
-                aim = fma2(ps, pv.im[p][cc], aim);
-              }
-              rv.re[p][cc] = fma2(ma, are, P == P16 ? mul2(rv.re[p][cc], rs) : rv.re[p][cc]);
-              rv.im[p][cc] = fma2(ma, aim, P == P16 ? mul2(rv.im[p][cc], rs) : rv.im[p][cc]);
-            }
-          nrm_sh[rhs * NT + threadIdx.x] += store_x2<P>(A.cg_r, i, rv);
+          nrm_sh[rhs * NT + threadIdx.x] += cg_epilogue_x2<P, CGR>(A, i, (float)cg_alpha[rhs], o);
         } else {
           const double n2 = store_x2<P>(A.out, i, o);
           if (NORM) nrm_sh[rhs * NT + threadIdx.x] += n2;
@@ -969,31 +1008,7 @@ __global__ void __launch_bounds__(NT, MINB) hop_kernel(DslashArgs A) {
     }
     }
   }
-  if (NORM || CGR) {
-    for (int q = 0; q < g.nrhs; q++) {
-      const double bs = block_sum<NT>(nrm_sh[q * NT + threadIdx.x], red);
-      if (threadIdx.x == 0) A.red.partial[q * gridDim.x + blockIdx.x] = bs;
-    }
-    if (last_block(A.red.ticket, gridDim.x)) {
-      __shared__ double total[MAX_RHS];
-      for (int q = 0; q < g.nrhs; q++) {
-        const double t = ordered_sum<NT>(A.red.partial + q * gridDim.x, gridDim.x, red);
-        if (threadIdx.x == 0) total[q] = t;
-      }
-      __syncthreads();
-      // the scalar steps of all right-hand sides side by side: each is a chain of
-      // global accesses of about 2 us
-      const int q = threadIdx.x;
-      if (q < g.nrhs && !(A.skip && A.skip[q])) {
-        if (!CGR) {
-          A.red.result[q] = total[q];
-        } else {
-          cg_advance(A.cg, q, total[q]);
-          if (A.red.result) A.red.result[q] = total[q];
-        }
-      }
-    }
-  }
+  if (NORM || CGR) hop_reduce<NT, CGR>(A, nrm_sh, red);
 }
 
 // ---------------------------------------------------------------- direction-parallel FP64 hop
@@ -1167,31 +1182,7 @@ __global__ void __launch_bounds__(NT) hop8_kernel(DslashArgs A) {
       if (NORM) nrm_sh[q * NT + threadIdx.x] += norm2(acc);
     }
   }
-  if (NORM || CGR) {
-    for (int q = 0; q < g.nrhs; q++) {
-      const double bs = block_sum<NT>(nrm_sh[q * NT + threadIdx.x], red);
-      if (threadIdx.x == 0) A.red.partial[q * gridDim.x + blockIdx.x] = bs;
-    }
-    if (last_block(A.red.ticket, gridDim.x)) {
-      __shared__ double total[MAX_RHS];
-      for (int q = 0; q < g.nrhs; q++) {
-        const double t = ordered_sum<NT>(A.red.partial + q * gridDim.x, gridDim.x, red);
-        if (threadIdx.x == 0) total[q] = t;
-      }
-      __syncthreads();
-      // the scalar steps of all right-hand sides side by side: each is a chain of
-      // global accesses of about 2 us
-      const int q = threadIdx.x;
-      if (q < g.nrhs && !(A.skip && A.skip[q])) {
-        if (!CGR) {
-          A.red.result[q] = total[q];
-        } else {
-          cg_advance(A.cg, q, total[q]);
-          if (A.red.result) A.red.result[q] = total[q];
-        }
-      }
-    }
-  }
+  if (NORM || CGR) hop_reduce<NT, CGR>(A, nrm_sh, red);
 }
 
 // Blocks of a kernel that fit on the device at once with this dynamic shared

@@ -5,7 +5,9 @@
 //   dag 0:  out = a * mix(M5^-1 (D in))                  (zmobius_m-sym2.h: the
 //           M5^-1 that follows the first kappa_b D4 of MatPc, dag 0)
 //   dag 1:  out = [x +] a * M5^-dag(mix^dag(D^dag in))  [, |out|^2]
-//           (zmobius_mdag-sym2.h: the M5^-dag after each D4^dag of MatPcDag)
+//           (zmobius_mdag-sym2.h: the M5^-dag after each D4^dag of MatPcDag), or
+//           with A.cg the CG update on it as in hop_kernel: out = A p is not stored
+//           but consumed by r -= alpha (A p + shift p), x += alpha p and |r|^2
 //
 // With 4-D checkerboarding (DWF_4D_EOPREC_EE) every slice of a site has the
 // same parity, so the column of a site holds all Ls slices and the block that
@@ -20,38 +22,36 @@
 
 namespace cpsb {
 
-// Element of the sweep tile: one complex component in the arithmetic type.
-template <int P> struct SweepT { typedef float2 T; typedef float R; };
-template <> struct SweepT<P64> { typedef double2 T; typedef double R; };
-
-// Dynamic shared memory: hop.cuh's tables, then the sweep tile of TX columns
-// x 12 components x (LS + 1) slots (the pad spreads the columns that one warp
-// sweeps over the banks).
+// Dynamic shared memory: hop.cuh's tables, then the sweep tile.
 template <int P, int LS>
 __host__ __device__ inline size_t hop_m5_tile_off(int TX, int NT, int nrhs, bool norm) {
   return (hop_shm(TX, NT, nrhs, norm, true).total + 15) & ~(size_t)15;
 }
 template <int P, int LS>
 __host__ __device__ inline size_t hop_m5_shm(int TX, int NT, int nrhs, bool norm) {
-  return hop_m5_tile_off<P, LS>(TX, NT, nrhs, norm) + (size_t)TX * 12 * (LS + 1) * sizeof(typename SweepT<P>::T);
+  return hop_m5_tile_off<P, LS>(TX, NT, nrhs, norm) + sweep_tile_bytes<P, LS>(TX);
 }
 
 // Thread t owns slice t % LS of tile column t / LS for every right-hand side
 // in turn; the skip mask is read per right-hand side, uniformly over the block,
 // so every thread reaches every barrier.
-template <int P, int NT, int MINB, bool DAG, bool XPAY, bool NORM, int LS, int DEPTH>
+template <int P, int NT, int MINB, bool DAG, bool XPAY, bool NORM, int CGR, int LS, int DEPTH>
 __global__ void __launch_bounds__(NT, MINB) hop_m5_kernel(DslashArgs A, M5Coef cf) {
   typedef typename SweepT<P>::T BT;
-  typedef typename SweepT<P>::R R;
   constexpr int TX = NT / LS;
   constexpr int CST = LS + 1;
   const Geom &g = A.g;
   extern __shared__ __align__(16) unsigned char dsh[];
   __shared__ double red[NT / 32];
-  const HopShm L = hop_shm(TX, NT, g.nrhs, NORM, true);
-  BT *tile_buf = (BT *)(dsh + hop_m5_tile_off<P, LS>(TX, NT, g.nrhs, NORM));
+  __shared__ double cg_alpha[MAX_RHS];  // as in hop_kernel
+  if (CGR && threadIdx.x < g.nrhs) {
+    const CgState *S = A.cg;
+    cg_alpha[threadIdx.x] = S->rr[threadIdx.x] / (S->d[threadIdx.x] + S->shift * S->pp[threadIdx.x]);
+  }
+  const HopShm L = hop_shm(TX, NT, g.nrhs, NORM || CGR, true);
+  BT *tile_buf = (BT *)(dsh + hop_m5_tile_off<P, LS>(TX, NT, g.nrhs, NORM || CGR));
   double *nrm_sh = (double *)(dsh + L.norm);
-  if (NORM)
+  if (NORM || CGR)
     for (int q = 0; q < g.nrhs; q++) nrm_sh[q * NT + threadIdx.x] = 0;
   const int sp = threadIdx.x % LS;
   const int xl = threadIdx.x / LS;
@@ -91,22 +91,8 @@ __global__ void __launch_bounds__(NT, MINB) hop_m5_kernel(DslashArgs A, M5Coef c
         }
       }
       __syncthreads();
-      // 2. the column operations, one thread per (column, component); the
-      // upper chirality (spins 0, 1) is q < 6 in both layouts.  Real
-      // coefficients act alike on the two members of a pair.
-      for (int t = threadIdx.x; t < nx * 12; t += NT) {
-        const int cx = t / 12, q = t - cx * 12;
-        BT *col = tile_buf + (size_t)(cx * 12 + q) * CST;
-        cplx<R> v[LS][1];
-#pragma unroll
-        for (int s = 0; s < LS; s++) v[s][0] = mk(col[s].x, col[s].y);
-        m5_column<LS, DAG ? 1 : 0, 1, R>(v, q < 6, cf);
-#pragma unroll
-        for (int s = 0; s < LS; s++) {
-          col[s].x = v[s][0].re;
-          col[s].y = v[s][0].im;
-        }
-      }
+      // 2. the column operations
+      sweep_tile<P, LS, DAG ? 1 : 0, NT>(tile_buf, nx, cf);
       __syncthreads();
       // 3. epilogue: out = [x +] a v
       if (act) {
@@ -124,8 +110,12 @@ __global__ void __launch_bounds__(NT, MINB) hop_m5_kernel(DslashArgs A, M5Coef c
 #pragma unroll
               for (int r = 0; r < 3; r++) o.c[s2][r] = xv.c[s2][r] + o.c[s2][r];
           }
-          store_spinor<P64>(A.out, i, o);
-          if (NORM) nrm_sh[rhs * NT + threadIdx.x] += norm2(o);
+          if (CGR) {
+            nrm_sh[rhs * NT + threadIdx.x] += cg_epilogue_64<CGR>(A, i, cg_alpha[rhs], o);
+          } else {
+            store_spinor<P64>(A.out, i, o);
+            if (NORM) nrm_sh[rhs * NT + threadIdx.x] += norm2(o);
+          }
         } else {
           const float2 a2 = f2b((float)A.a);
           SpX2 o;
@@ -146,37 +136,31 @@ __global__ void __launch_bounds__(NT, MINB) hop_m5_kernel(DslashArgs A, M5Coef c
                 o.im[p][cc] = fma2(xv.im[p][cc], xs, o.im[p][cc]);
               }
           }
-          const double n2 = store_x2<P>(A.out, i, o);
-          if (NORM) nrm_sh[rhs * NT + threadIdx.x] += n2;
+          if (CGR) {
+            nrm_sh[rhs * NT + threadIdx.x] += cg_epilogue_x2<P, CGR>(A, i, (float)cg_alpha[rhs], o);
+          } else {
+            const double n2 = store_x2<P>(A.out, i, o);
+            if (NORM) nrm_sh[rhs * NT + threadIdx.x] += n2;
+          }
         }
       }
       __syncthreads();  // every entry is read back before the next right-hand side's hop
     }
   }
-  if (NORM) {
-    for (int q = 0; q < g.nrhs; q++) {
-      const double bs = block_sum<NT>(nrm_sh[q * NT + threadIdx.x], red);
-      if (threadIdx.x == 0) A.red.partial[q * gridDim.x + blockIdx.x] = bs;
-    }
-    if (last_block(A.red.ticket, gridDim.x)) {
-      for (int q = 0; q < g.nrhs; q++) {
-        const double t = ordered_sum<NT>(A.red.partial + q * gridDim.x, gridDim.x, red);
-        if (threadIdx.x == 0 && !(A.skip && A.skip[q])) A.red.result[q] = t;
-        __syncthreads();
-      }
-    }
-  }
+  if (NORM || CGR) hop_reduce<NT, CGR>(A, nrm_sh, red);
 }
 
-template <int P, int LS, bool DAG, bool XPAY, bool NORM>
+template <int P, int LS, bool DAG, bool XPAY, bool NORM, int CGR>
 static cudaError_t hop_m5_launch_m(const DslashArgs &A, const M5Coef &cf, cudaStream_t st) {
   constexpr int NT = 128;
-  constexpr int MINB = P == P64 ? 2 : 4;
+  // FP64: 168 registers for 12 warps an SM; with 255 for 8 the hops of 24^3x64, Ls 16 took
+  // 1515, 1375 and 1354 us, now 1330, 1317 and 1310
+  constexpr int MINB = P == P64 ? 3 : 4;
   constexpr int DEPTH = P == P64 ? 1 : 2;
   constexpr int TX = NT / LS;
-  const size_t shm = hop_m5_shm<P, LS>(TX, NT, A.g.nrhs, NORM);
+  const size_t shm = hop_m5_shm<P, LS>(TX, NT, A.g.nrhs, NORM || CGR);
   if (shm > 200 * 1024) return cudaErrorNotSupported;
-  const void *fn = (const void *)hop_m5_kernel<P, NT, MINB, DAG, XPAY, NORM, LS, DEPTH>;
+  const void *fn = (const void *)hop_m5_kernel<P, NT, MINB, DAG, XPAY, NORM, CGR, LS, DEPTH>;
   static bool opted = false;
   if (!opted && shm + 1024 > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
@@ -185,20 +169,25 @@ static cudaError_t hop_m5_launch_m(const DslashArgs &A, const M5Coef &cf, cudaSt
   }
   const long ntiles = (A.g.n4cb + TX - 1) / TX;
   const long nb = std::min(ntiles, (long)resident_blocks(fn, NT, shm));
-  hop_m5_kernel<P, NT, MINB, DAG, XPAY, NORM, LS, DEPTH><<<(unsigned)nb, NT, shm, st>>>(A, cf);
+  hop_m5_kernel<P, NT, MINB, DAG, XPAY, NORM, CGR, LS, DEPTH><<<(unsigned)nb, NT, shm, st>>>(A, cf);
   return launched();
 }
 
 template <int P, int LS>
 static cudaError_t hop_m5_launch_ls(const DslashArgs &A, const M5Coef &cf, int xpay, int norm, cudaStream_t st) {
+  if (A.cg) {  // the CG residual update: dag 1, xpay
+    if (!A.dag || !xpay || !A.cg_x.data) return cudaErrorInvalidValue;
+    if (A.cg_shift) return hop_m5_launch_m<P, LS, true, true, false, 2>(A, cf, st);
+    return hop_m5_launch_m<P, LS, true, true, false, 1>(A, cf, st);
+  }
   if (!A.dag) {
     if (xpay || norm) return cudaErrorNotSupported;
-    return hop_m5_launch_m<P, LS, false, false, false>(A, cf, st);
+    return hop_m5_launch_m<P, LS, false, false, false, 0>(A, cf, st);
   }
-  if (xpay && norm) return hop_m5_launch_m<P, LS, true, true, true>(A, cf, st);
-  if (xpay) return hop_m5_launch_m<P, LS, true, true, false>(A, cf, st);
+  if (xpay && norm) return hop_m5_launch_m<P, LS, true, true, true, 0>(A, cf, st);
+  if (xpay) return hop_m5_launch_m<P, LS, true, true, false, 0>(A, cf, st);
   if (norm) return cudaErrorNotSupported;
-  return hop_m5_launch_m<P, LS, true, false, false>(A, cf, st);
+  return hop_m5_launch_m<P, LS, true, false, false, 0>(A, cf, st);
 }
 
 // The fused hop + M5 for one storage precision; cudaErrorNotSupported for a
@@ -206,7 +195,7 @@ static cudaError_t hop_m5_launch_ls(const DslashArgs &A, const M5Coef &cf, int x
 // Ls not listed), for which the caller runs the hop and the M5 kernel.
 template <int P>
 static cudaError_t hop_m5_launch_p(const DslashArgs &A, const M5Coef &cf, int xpay, int norm, cudaStream_t st) {
-  if (A.five_d || A.hop5 || A.g.ncls != 1 || A.g.cs[0] != A.g.ls || A.cg) return cudaErrorNotSupported;
+  if (A.five_d || A.hop5 || A.g.ncls != 1 || A.g.cs[0] != A.g.ls) return cudaErrorNotSupported;
   switch (A.g.ls) {
     case 4: return hop_m5_launch_ls<P, 4>(A, cf, xpay, norm, st);
     case 8: return hop_m5_launch_ls<P, 8>(A, cf, xpay, norm, st);

@@ -187,11 +187,14 @@ struct Operator {
     mdagm(out.ptr(), in.ptr(), red, skip, st);
   }
   // MatPcDagMatPc p with the CG residual update fused into its last hop
-  // (Wilson / DWF, every precision): |MatPc p|^2 -> red_d, then
+  // (Wilson, DWF and Mobius SYM2, every precision): |MatPc p|^2 -> red_d, then
   // r -= alpha (A p + shift p), |r|^2 and the recurrence scalars in S, and
   // x += alpha p; A p is not stored (scratch receives it only while a
   // launch shape is being tuned).
-  bool can_fuse_cg_r() const { return p.action == CPSB_WILSON || p.action == CPSB_DWF; }
+  bool can_fuse_cg_r() const {
+    return p.action == CPSB_WILSON || p.action == CPSB_DWF ||
+           (p.action == CPSB_MOBIUS && p.pc_type == 2 && fuse_m5);
+  }
   bool mobius_like() const { return p.action == CPSB_MOBIUS || p.action == CPSB_ZMOBIUS; }
   void matpc_zmobius(const SpinorPtr &out, const SpinorPtr &in, int dag, const Reduce *red, const int *skip,
                      cudaStream_t st);

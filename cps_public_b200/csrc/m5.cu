@@ -24,6 +24,7 @@
 #include <string.h>
 
 #include "blas.h"
+#include "hop.cuh"
 #include "m5_sweep.cuh"
 
 namespace cpsb {
@@ -138,11 +139,127 @@ __device__ __forceinline__ void m5z_column(cplx<T> (&v)[LS][NC], int h, const ZM
 // Sites per tile of the tiled kernels: one sweep thread per (site, chunk).
 template <int P, int NT> struct M5Tile { static const int TX = NT / ChunkT<P>::NCH; };
 
-// The tiled kernel: Z = false applies m5_column with the real coefficients cf,
-// Z = true m5z_column with the table tab.  out = [x +] sc * v (sc = cf.scale
-// for Z = false, 1 for Z = true).
-template <int P, int LS, int DAG, bool XPAY, bool NORM, int NT, bool Z>
-__global__ void __launch_bounds__(NT) m5t_kernel(Geom g, SpinorPtr out, SpinorPtr in, SpinorPtr xv, M5Coef cf,
+// The real-coefficient kernel: out = [x +] scale * v, v the column operations.  A
+// block takes TX = NT / LS whole columns, a thread per entry, through the sweep
+// tile of m5_sweep.cuh, whose rows a warp reads and writes without bank conflicts
+// (whole spinors in shared memory, 192 bytes apart, cost 4 wavefronts for 1).  24^3x64, Ls 16, FP64: 630 -> 420 us (6.5 TB/s);
+// 16^3x32, Ls 12, 16-bit, 4 right-hand sides: 105 -> 73 us.
+template <int P, int LS, int DAG, bool XPAY, bool NORM, int NT>
+__global__ void __launch_bounds__(NT) m5_kernel(Geom g, SpinorPtr out, SpinorPtr in, SpinorPtr xv, M5Coef cf,
+                                                Reduce red, const int *skip) {
+  typedef typename SweepT<P>::T BT;
+  constexpr int TX = NT / LS, CST = LS + 1;
+  extern __shared__ __align__(16) unsigned char m5sh[];
+  BT *buf = (BT *)m5sh;
+  __shared__ double sh[NT / 32];
+  const int rhs = blockIdx.y;
+  const unsigned per = (unsigned)g.n4cb * (unsigned)LS;
+  const int ntiles = (g.n4cb + TX - 1) / TX;
+  BT *mine = buf + (size_t)(threadIdx.x / LS) * 12 * CST + threadIdx.x % LS;
+  double acc = 0;
+  const bool sk = skip && skip[rhs];
+  for (int tile = blockIdx.x; !sk && tile < ntiles; tile += gridDim.x) {
+    const int nx = min(TX, g.n4cb - tile * TX);
+    const bool act = (int)threadIdx.x < nx * LS;
+    const unsigned i = (unsigned)rhs * per + (unsigned)tile * (unsigned)(TX * LS) + threadIdx.x;
+    // a thread's own slots between tiles: read back below, written here
+    if (act) {
+      if constexpr (P == P64) {
+        const Raw<P64> r = load_raw<P64>(in, i);
+#pragma unroll
+        for (int q = 0; q < 12; q++) mine[q * CST] = r.c[q];
+      } else {
+        float nrm;
+        const SpX2 s = unpack(load_raw<P>(in, i), &nrm);
+        const float2 n2 = f2b(nrm);
+#pragma unroll
+        for (int q = 0; q < 6; q++) {
+          mine[(2 * q) * CST] = P == P16 ? mul2(n2, s.re[q / 3][q % 3]) : s.re[q / 3][q % 3];
+          mine[(2 * q + 1) * CST] = P == P16 ? mul2(n2, s.im[q / 3][q % 3]) : s.im[q / 3][q % 3];
+        }
+      }
+    }
+    __syncthreads();
+    sweep_tile<P, LS, DAG, NT>(buf, nx, cf);
+    __syncthreads();
+    if (act) {
+      if constexpr (P == P64) {
+        const double sc = cf.scale;
+        Spinor<double> o;
+#pragma unroll
+        for (int q = 0; q < 12; q++) o.c[q / 3][q % 3] = mk(sc * mine[q * CST].x, sc * mine[q * CST].y);
+        if (XPAY) {
+          const Spinor<double> xo = unpack64(load_raw<P64>(xv, i));
+#pragma unroll
+          for (int q = 0; q < 12; q++) o.c[q / 3][q % 3] = xo.c[q / 3][q % 3] + o.c[q / 3][q % 3];
+        }
+        store_spinor<P64>(out, i, o);
+        if (NORM) acc += norm2(o);
+      } else {
+        const float2 sc = f2b((float)cf.scale);
+        SpX2 o;
+#pragma unroll
+        for (int q = 0; q < 6; q++) {
+          o.re[q / 3][q % 3] = mul2(sc, mine[(2 * q) * CST]);
+          o.im[q / 3][q % 3] = mul2(sc, mine[(2 * q + 1) * CST]);
+        }
+        if (XPAY) {
+          float xn;
+          const SpX2 xo = unpack(load_raw<P>(xv, i), &xn);
+          const float2 xs = f2b(xn);
+#pragma unroll
+          for (int p = 0; p < 2; p++)
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+              o.re[p][c] = fma2(xo.re[p][c], xs, o.re[p][c]);
+              o.im[p][c] = fma2(xo.im[p][c], xs, o.im[p][c]);
+            }
+        }
+        const double n2 = store_x2<P>(out, i, o);
+        if (NORM) acc += n2;
+      }
+    }
+  }
+  if (NORM) m5_norm_epilogue<NT>(acc, g, red, skip, sh);
+}
+
+template <int P, int LS>
+static cudaError_t m5_launch(int dag, const Geom &g, SpinorPtr out, SpinorPtr in, SpinorPtr x, const M5Coef &cf,
+                             int xpay, int norm, Reduce red, const int *skip, cudaStream_t st) {
+  constexpr int NT = 128, TX = NT / LS;
+  if (g.ncls != 1 || g.ls != LS) return cudaErrorInvalidValue;
+  const size_t shm = sweep_tile_bytes<P, LS>(TX);  // at most 31 KB
+  const int ntiles = (g.n4cb + TX - 1) / TX;
+  const dim3 grid(ntiles < 148 * 16 ? ntiles : 148 * 16, g.nrhs);
+#define CPSB_M5(D, XP, NR)                                                                  \
+  if (dag == D && !!xpay == XP && !!norm == NR) {                                           \
+    m5_kernel<P, LS, D, XP, NR, NT><<<grid, NT, shm, st>>>(g, out, in, x, cf, red, skip);   \
+    return launched();                                                                      \
+  }
+  CPSB_M5(0, false, false) CPSB_M5(0, true, false) CPSB_M5(0, true, true) CPSB_M5(0, false, true)
+  CPSB_M5(1, false, false) CPSB_M5(1, true, false) CPSB_M5(1, true, true) CPSB_M5(1, false, true)
+#undef CPSB_M5
+  return cudaErrorInvalidValue;
+}
+
+template <int P>
+static cudaError_t m5_launch_p(int dag, const Geom &g, SpinorPtr out, SpinorPtr in, SpinorPtr x, const M5Coef &cf,
+                               int xpay, int norm, Reduce red, const int *skip, cudaStream_t st) {
+  switch (g.ls) {
+    case 4: return m5_launch<P, 4>(dag, g, out, in, x, cf, xpay, norm, red, skip, st);
+    case 8: return m5_launch<P, 8>(dag, g, out, in, x, cf, xpay, norm, red, skip, st);
+    case 12: return m5_launch<P, 12>(dag, g, out, in, x, cf, xpay, norm, red, skip, st);
+    case 16: return m5_launch<P, 16>(dag, g, out, in, x, cf, xpay, norm, red, skip, st);
+    case 20: return m5_launch<P, 20>(dag, g, out, in, x, cf, xpay, norm, red, skip, st);
+    case 24: return m5_launch<P, 24>(dag, g, out, in, x, cf, xpay, norm, red, skip, st);
+    case 32: return m5_launch<P, 32>(dag, g, out, in, x, cf, xpay, norm, red, skip, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+// The zMobius kernel: out = [x +] v, m5z_column with the table tab.
+template <int P, int LS, int DAG, bool XPAY, bool NORM, int NT>
+__global__ void __launch_bounds__(NT) m5t_kernel(Geom g, SpinorPtr out, SpinorPtr in, SpinorPtr xv,
                                                  const ZM5Tab *tab, Reduce red, const int *skip) {
   typedef typename ChunkT<P>::T T;
   constexpr int NCH = ChunkT<P>::NCH, NC = ChunkT<P>::NC, TX = M5Tile<P, NT>::TX;
@@ -152,7 +269,6 @@ __global__ void __launch_bounds__(NT) m5t_kernel(Geom g, SpinorPtr out, SpinorPt
   const int rhs = blockIdx.y;
   const long per = (long)g.n4cb * LS;
   const int ntiles = (g.n4cb + TX - 1) / TX;
-  const T sc = Z ? T(1) : (T)cf.scale;
   double acc = 0;
   const bool sk = skip && skip[rhs];
   for (int tile = blockIdx.x; !sk && tile < ntiles; tile += gridDim.x) {
@@ -168,8 +284,7 @@ __global__ void __launch_bounds__(NT) m5t_kernel(Geom g, SpinorPtr out, SpinorPt
       for (int s = 0; s < LS; s++)
 #pragma unroll
         for (int q = 0; q < NC; q++) v[s][q] = chunk_elem<NC>(buf[xl * LS + s], k, q);
-      if (Z) m5z_column<LS, DAG, NC, T>(v, k < NCH / 2 ? 0 : 1, tab);
-      else m5_column<LS, DAG, NC, T>(v, k < NCH / 2, cf);
+      m5z_column<LS, DAG, NC, T>(v, k < NCH / 2 ? 0 : 1, tab);
 #pragma unroll
       for (int s = 0; s < LS; s++)
 #pragma unroll
@@ -183,12 +298,7 @@ __global__ void __launch_bounds__(NT) m5t_kernel(Geom g, SpinorPtr out, SpinorPt
 #pragma unroll
         for (int a = 0; a < 4; a++)
 #pragma unroll
-          for (int c = 0; c < 3; c++) o.c[a][c] = xo.c[a][c] + cscale(sc, o.c[a][c]);
-      } else if (!Z) {
-#pragma unroll
-        for (int a = 0; a < 4; a++)
-#pragma unroll
-          for (int c = 0; c < 3; c++) o.c[a][c] = cscale(sc, o.c[a][c]);
+          for (int c = 0; c < 3; c++) o.c[a][c] = xo.c[a][c] + o.c[a][c];
       }
       store_spinor<P>(out, base + t, o);
       if (NORM) acc += norm2(rounded<P>(o));
@@ -197,8 +307,8 @@ __global__ void __launch_bounds__(NT) m5t_kernel(Geom g, SpinorPtr out, SpinorPt
   if (NORM) m5_norm_epilogue<NT>(acc, g, red, skip, sh);
 }
 
-template <int P, int LS, bool Z>
-static cudaError_t m5t_launch(int dag, const Geom &g, SpinorPtr out, SpinorPtr in, SpinorPtr x, const M5Coef &cf,
+template <int P, int LS>
+static cudaError_t m5t_launch(int dag, const Geom &g, SpinorPtr out, SpinorPtr in, SpinorPtr x,
                               const ZM5Tab *tab, int xpay, int norm, Reduce red, const int *skip, cudaStream_t st) {
   constexpr int NT = 128;
   typedef typename ChunkT<P>::T T;
@@ -211,12 +321,12 @@ static cudaError_t m5t_launch(int dag, const Geom &g, SpinorPtr out, SpinorPtr i
   if (dag == D && !!xpay == XP && !!norm == NR) {                                                      \
     static bool attr = false;                                                                          \
     if (!attr && shm > 48 * 1024) {                                                                    \
-      const cudaError_t e = cudaFuncSetAttribute((const void *)m5t_kernel<P, LS, D, XP, NR, NT, Z>,    \
+      const cudaError_t e = cudaFuncSetAttribute((const void *)m5t_kernel<P, LS, D, XP, NR, NT>,    \
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm); \
       if (e != cudaSuccess) return e;                                                                  \
       attr = true;                                                                                     \
     }                                                                                                  \
-    m5t_kernel<P, LS, D, XP, NR, NT, Z><<<grid, NT, shm, st>>>(g, out, in, x, cf, tab, red, skip);     \
+    m5t_kernel<P, LS, D, XP, NR, NT><<<grid, NT, shm, st>>>(g, out, in, x, tab, red, skip);           \
     return launched();                                                                                 \
   }
   CPSB_M5T(0, false, false) CPSB_M5T(0, true, false) CPSB_M5T(0, true, true) CPSB_M5T(0, false, true)
@@ -225,37 +335,35 @@ static cudaError_t m5t_launch(int dag, const Geom &g, SpinorPtr out, SpinorPtr i
   return cudaErrorInvalidValue;
 }
 
-template <int P, bool Z>
-static cudaError_t m5t_launch_p(int dag, const Geom &g, SpinorPtr out, SpinorPtr in, SpinorPtr x, const M5Coef &cf,
+template <int P>
+static cudaError_t m5t_launch_p(int dag, const Geom &g, SpinorPtr out, SpinorPtr in, SpinorPtr x,
                                 const ZM5Tab *tab, int xpay, int norm, Reduce red, const int *skip,
                                 cudaStream_t st) {
   switch (g.ls) {
-    case 4: return m5t_launch<P, 4, Z>(dag, g, out, in, x, cf, tab, xpay, norm, red, skip, st);
-    case 8: return m5t_launch<P, 8, Z>(dag, g, out, in, x, cf, tab, xpay, norm, red, skip, st);
-    case 12: return m5t_launch<P, 12, Z>(dag, g, out, in, x, cf, tab, xpay, norm, red, skip, st);
-    case 16: return m5t_launch<P, 16, Z>(dag, g, out, in, x, cf, tab, xpay, norm, red, skip, st);
-    case 20: return m5t_launch<P, 20, Z>(dag, g, out, in, x, cf, tab, xpay, norm, red, skip, st);
-    case 24: return m5t_launch<P, 24, Z>(dag, g, out, in, x, cf, tab, xpay, norm, red, skip, st);
-    case 32: return m5t_launch<P, 32, Z>(dag, g, out, in, x, cf, tab, xpay, norm, red, skip, st);
+    case 4: return m5t_launch<P, 4>(dag, g, out, in, x, tab, xpay, norm, red, skip, st);
+    case 8: return m5t_launch<P, 8>(dag, g, out, in, x, tab, xpay, norm, red, skip, st);
+    case 12: return m5t_launch<P, 12>(dag, g, out, in, x, tab, xpay, norm, red, skip, st);
+    case 16: return m5t_launch<P, 16>(dag, g, out, in, x, tab, xpay, norm, red, skip, st);
+    case 20: return m5t_launch<P, 20>(dag, g, out, in, x, tab, xpay, norm, red, skip, st);
+    case 24: return m5t_launch<P, 24>(dag, g, out, in, x, tab, xpay, norm, red, skip, st);
+    case 32: return m5t_launch<P, 32>(dag, g, out, in, x, tab, xpay, norm, red, skip, st);
     default: return cudaErrorInvalidValue;
   }
 }
 
 cudaError_t launch_m5(int prec, int dag, const Geom &g, SpinorPtr out, SpinorPtr in, SpinorPtr x, const M5Coef &cf,
                       int xpay, int norm, Reduce red, const int *skip, cudaStream_t st) {
-  if (prec == P64) return m5t_launch_p<P64, false>(dag, g, out, in, x, cf, nullptr, xpay, norm, red, skip, st);
-  if (prec == P32) return m5t_launch_p<P32, false>(dag, g, out, in, x, cf, nullptr, xpay, norm, red, skip, st);
-  if (prec == P16) return m5t_launch_p<P16, false>(dag, g, out, in, x, cf, nullptr, xpay, norm, red, skip, st);
+  if (prec == P64) return m5_launch_p<P64>(dag, g, out, in, x, cf, xpay, norm, red, skip, st);
+  if (prec == P32) return m5_launch_p<P32>(dag, g, out, in, x, cf, xpay, norm, red, skip, st);
+  if (prec == P16) return m5_launch_p<P16>(dag, g, out, in, x, cf, xpay, norm, red, skip, st);
   return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_m5z(int prec, int dag, const Geom &g, SpinorPtr out, SpinorPtr in, SpinorPtr x,
                        const ZM5Tab *tab, int xpay, int norm, Reduce red, const int *skip, cudaStream_t st) {
-  M5Coef none;
-  memset(&none, 0, sizeof(none));
-  if (prec == P64) return m5t_launch_p<P64, true>(dag, g, out, in, x, none, tab, xpay, norm, red, skip, st);
-  if (prec == P32) return m5t_launch_p<P32, true>(dag, g, out, in, x, none, tab, xpay, norm, red, skip, st);
-  if (prec == P16) return m5t_launch_p<P16, true>(dag, g, out, in, x, none, tab, xpay, norm, red, skip, st);
+  if (prec == P64) return m5t_launch_p<P64>(dag, g, out, in, x, tab, xpay, norm, red, skip, st);
+  if (prec == P32) return m5t_launch_p<P32>(dag, g, out, in, x, tab, xpay, norm, red, skip, st);
+  if (prec == P16) return m5t_launch_p<P16>(dag, g, out, in, x, tab, xpay, norm, red, skip, st);
   return cudaErrorInvalidValue;
 }
 

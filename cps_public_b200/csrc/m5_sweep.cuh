@@ -82,4 +82,44 @@ __device__ __forceinline__ void m5_column(cplx<T> (&v)[LS][NC], bool upper, cons
   if (DAG == 0) mix_inplace<LS, NC, T>(v, upper, b, c, mwall);
 }
 
+// Element of a sweep tile: one complex component (FP64: q = 3 spin + colour as
+// (re, im); FP32 / 16-bit: q = 2 (3 p + colour) + (0 re, 1 im) as the lanes
+// (spin 2p, spin 2p + 1)).  Component q of slice s of tile column xl sits at
+// (xl * 12 + q) * (LS + 1) + s: the pad spreads the columns that one warp sweeps over
+// the banks.
+template <int P> struct SweepT { typedef float2 T; typedef float R; };
+template <> struct SweepT<P64> { typedef double2 T; typedef double R; };
+template <int P, int LS>
+__host__ __device__ inline size_t sweep_tile_bytes(int TX) {
+  return (size_t)TX * 12 * (LS + 1) * sizeof(typename SweepT<P>::T);
+}
+
+// m5_column on every column of a tile of nx columns, one thread per (column,
+// component).  The chiralities (components q < 6 and q >= 6 in both layouts) take
+// their sweeps in opposite orders, so each half of the components starts on a warp
+// boundary: no warp runs both (Mobius 16^3x32, Ls 12, 16-bit, 4 right-hand sides: the two
+// hops with M5 inside 236 and 227 -> 206 us).
+template <int P, int LS, int DAG, int NT>
+__device__ __forceinline__ void sweep_tile(typename SweepT<P>::T *tile, int nx, const M5Coef &cf) {
+  typedef typename SweepT<P>::R R;
+  const int half = nx * 6, pad = (half + 31) & ~31;
+  for (int t = threadIdx.x; t < 2 * pad; t += NT) {
+    const bool upper = t < pad;
+    const int u = upper ? t : t - pad;
+    if (u >= half) continue;
+    const int cx = u / 6, q = u - cx * 6 + (upper ? 0 : 6);
+    typename SweepT<P>::T *col = tile + (size_t)(cx * 12 + q) * (LS + 1);
+    // real coefficients act alike on the two members of a pair
+    cplx<R> v[LS][1];
+#pragma unroll
+    for (int s = 0; s < LS; s++) v[s][0] = mk(col[s].x, col[s].y);
+    m5_column<LS, DAG, 1, R>(v, upper, cf);
+#pragma unroll
+    for (int s = 0; s < LS; s++) {
+      col[s].x = v[s][0].re;
+      col[s].y = v[s][0].im;
+    }
+  }
+}
+
 }  // namespace cpsb

@@ -819,15 +819,20 @@ void Operator::mobius_hop5_add(const SpinorPtr &out, const SpinorPtr &in, const 
 void Operator::mdagm_cg_r(const SpinorPtr &scratch, const SpinorPtr &in, const Reduce *red_d, const int *skip,
                           CgState *S, const SpinorPtr &r, const Reduce *red_r, bool shifted, const SpinorPtr &x,
                           cudaStream_t st) {
-  if (!can_fuse_cg_r()) throw Error{CPSB_ERR_UNSUPPORTED, "fused residual update needs the Wilson or DWF operator"};
+  if (!can_fuse_cg_r())
+    throw Error{CPSB_ERR_UNSUPPORTED, "fused residual update: Wilson, DWF and Mobius SYM2 operators"};
   matpc(t2.ptr(), in, 0, red_d, skip, st);  // |MatPc p|^2 -> d
-  hop(t1.ptr(), t2.ptr(), 1, 1, 1.0, nullptr, nullptr, skip, st);
-  // the last hop of MatPcDag: out = t2 - kappa^2 D t1 = A p, consumed in registers
+  const bool mob = p.action == CPSB_MOBIUS;
+  if (!mob) hop(t1.ptr(), t2.ptr(), 1, 1, 1.0, nullptr, nullptr, skip, st);
+  else if (!hop_m5(t3.ptr(), t2.ptr(), 1, 1, -kappa_b * kappa_b, m5c[1], nullptr, nullptr, skip, st))
+    throw Error{CPSB_ERR_UNSUPPORTED, "no fused hop + M5 kernel for this operator"};
+  // the last hop of MatPcDag: out = t2 - kappa^2 D t1 (Mobius: t2 + M5^-dag mix^dag D t3)
+  // = A p, consumed in registers
   DslashArgs A;
   memset(&A, 0, sizeof(A));
   A.g = geom;
   A.U = G->ptr(prec);
-  A.in = t1.ptr();
+  A.in = mob ? t3.ptr() : t1.ptr();
   A.out = scratch;
   A.x = t2.ptr();
   A.cb = 0;
@@ -836,18 +841,19 @@ void Operator::mdagm_cg_r(const SpinorPtr &scratch, const SpinorPtr &in, const R
   A.hop5 = p.action == CPSB_DWF;
   A.hop5_fact = 2.0 * p.a5_inv;
   A.hop5_wall = -2.0 * p.mass * p.a5_inv;
-  A.a = -kappa * kappa;
-  A.bc_t_sign = G->bc_t ? -1.0 : 1.0;
+  A.a = mob ? m5c[1].scale : -kappa * kappa;
+  A.bc_t_sign = (prec != P64 && G->bc_t) ? -1.0 : 1.0;
   A.skip = skip;
   // launch shape of the same hop without the fused update (tuned on the scratch output)
-  const int v = tuned_variant(A, prec, 1, 0, st);
+  const int v = mob ? 0 : tuned_variant(A, prec, 1, 0, st);
   A.red = *red_r;
   A.cg = S;
   A.cg_r = r;
   A.cg_p = in;
   A.cg_shift = shifted ? 1 : 0;
   A.cg_x = x;
-  CK(launch_dslash(prec, A, 1, 1, v, st));
+  if (mob) CK(launch_hop_m5(prec, A, m5c[1], 1, 0, st));
+  else CK(launch_dslash(prec, A, 1, 1, v, st));
 }
 
 void Operator::mdagm(const SpinorPtr &out, const SpinorPtr &in, const Reduce *red, const int *skip, cudaStream_t st) {
