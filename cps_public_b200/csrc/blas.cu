@@ -245,6 +245,10 @@ template <int P, int NT>
 __global__ void __launch_bounds__(NT) cg_r_update_kernel(Geom g, SpinorPtr r, SpinorPtr Ap, SpinorPtr p, CgState *S, Reduce red) {
   typedef typename PrecTraits<P>::real T;
   __shared__ double sh[NT / 32];
+  if (P == P64) {
+    grid_wait();
+    grid_release();
+  }
   const int rhs = blockIdx.y;
   const long per = (long)g.n4cb * g.ls;
   double acc = 0;
@@ -306,6 +310,10 @@ __global__ void __launch_bounds__(NT) cg_xp_update_kernel(Geom g, SpinorPtr x, S
   typedef typename PrecTraits<P>::real T;
   typedef typename PrecTraits<PX>::real TX;
   __shared__ double sh[NT / 32];
+  if (P == P64) {
+    grid_wait();
+    grid_release();
+  }
   const int rhs = blockIdx.y;
   const long per = (long)g.n4cb * g.ls;
   const bool want_pp = S->shift != 0.0;
@@ -356,20 +364,18 @@ __global__ void __launch_bounds__(NT) cg_xp_update_kernel(Geom g, SpinorPtr x, S
 cudaError_t launch_cg_r_update(int prec, const Geom &g, SpinorPtr r, SpinorPtr Ap, SpinorPtr p, CgState *S, Reduce red,
                                cudaStream_t st) {
   dim3 grid(grid_blocks((long)g.n4cb * g.ls, 256), g.nrhs);
-  if (prec == P64) cg_r_update_kernel<P64, 256><<<grid, 256, 0, st>>>(g, r, Ap, p, S, red);
-  else if (prec == P32) cg_r_update_kernel<P32, 256><<<grid, 256, 0, st>>>(g, r, Ap, p, S, red);
-  else cg_r_update_kernel<P16, 256><<<grid, 256, 0, st>>>(g, r, Ap, p, S, red);
-  return launched();
+  if (prec == P64) return launch_chained<P64>(cg_r_update_kernel<P64, 256>, grid, 256, 0, st, g, r, Ap, p, S, red);
+  else if (prec == P32) return launch_chained<P32>(cg_r_update_kernel<P32, 256>, grid, 256, 0, st, g, r, Ap, p, S, red);
+  else return launch_chained<P16>(cg_r_update_kernel<P16, 256>, grid, 256, 0, st, g, r, Ap, p, S, red);
 }
 
 cudaError_t launch_cg_xp_update(int px, int prec, const Geom &g, SpinorPtr x, SpinorPtr p, SpinorPtr r, CgState *S,
                                 Reduce red, cudaStream_t st) {
   dim3 grid(grid_blocks((long)g.n4cb * g.ls, 256), g.nrhs);
-  if (px == P64 && prec == P64) cg_xp_update_kernel<P64, P64, 256><<<grid, 256, 0, st>>>(g, x, p, r, S, red);
-  else if (px == P32 && prec == P32) cg_xp_update_kernel<P32, P32, 256><<<grid, 256, 0, st>>>(g, x, p, r, S, red);
-  else if (px == P32 && prec == P16) cg_xp_update_kernel<P32, P16, 256><<<grid, 256, 0, st>>>(g, x, p, r, S, red);
-  else return cudaErrorInvalidValue;
-  return launched();
+  if (px == P64 && prec == P64) return launch_chained<P64>(cg_xp_update_kernel<P64, P64, 256>, grid, 256, 0, st, g, x, p, r, S, red);
+  else if (px == P32 && prec == P32) return launch_chained<P32>(cg_xp_update_kernel<P32, P32, 256>, grid, 256, 0, st, g, x, p, r, S, red);
+  else if (px == P32 && prec == P16) return launch_chained<P16>(cg_xp_update_kernel<P32, P16, 256>, grid, 256, 0, st, g, x, p, r, S, red);
+  return cudaErrorInvalidValue;
 }
 
 // ---------------------------------------------------------------- axpby
@@ -381,6 +387,10 @@ __global__ void __launch_bounds__(NT) axpby_kernel(Geom g, SpinorPtr out, Spinor
   typedef typename PrecTraits<PO>::real TO;
   typedef double TA;
   __shared__ double sh[NT / 32];
+  if (PO == P64 && PX == P64 && PY == P64) {
+    grid_wait();
+    grid_release();
+  }
   const int rhs = blockIdx.y;
   const long per = (long)g.n4cb * g.ls;
   double acc = 0;
@@ -425,8 +435,8 @@ cudaError_t launch_axpby(int po, SpinorPtr out, int px, SpinorPtr X, int py, Spi
   dim3 grid(grid_blocks((long)g.n4cb * g.ls, 256), g.nrhs);
 #define AX(A, B, C)                                                                               \
   if (po == A && px == B && py == C) {                                                          \
-    axpby_kernel<A, B, C, 256><<<grid, 256, 0, st>>>(g, out, X, Y, sc, skip, red, norm);        \
-    return launched();                                                                  \
+    return launch_chained<(A == P64 && B == P64 && C == P64) ? P64 : P32>(axpby_kernel<A, B, C, 256>, grid, 256, 0, st, g, \
+                                                                          out, X, Y, sc, skip, red, norm);                  \
   }
   AX(P64, P64, P64) AX(P64, P64, P32) AX(P64, P32, P64) AX(P64, P16, P64) AX(P64, P64, P16)
   AX(P32, P32, P32) AX(P32, P64, P32) AX(P32, P32, P64) AX(P32, P16, P32) AX(P32, P32, P16)
@@ -441,6 +451,10 @@ template <int P, int NT>
 __global__ void __launch_bounds__(NT) redot_kernel(Geom g, SpinorPtr X, SpinorPtr Y, Reduce red) {
   typedef typename PrecTraits<P>::real T;
   __shared__ double sh[NT / 32];
+  if (P == P64) {
+    grid_wait();
+    grid_release();
+  }
   const int rhs = blockIdx.y;
   const long per = (long)g.n4cb * g.ls;
   double acc = 0;
@@ -512,10 +526,9 @@ cudaError_t launch_caxpy(SpinorPtr out, double cr, double ci, SpinorPtr X, Spino
 
 cudaError_t launch_redot(int prec, const Geom &g, SpinorPtr X, SpinorPtr Y, Reduce red, cudaStream_t st) {
   dim3 grid(grid_blocks((long)g.n4cb * g.ls, 256), g.nrhs);
-  if (prec == P64) redot_kernel<P64, 256><<<grid, 256, 0, st>>>(g, X, Y, red);
-  else if (prec == P32) redot_kernel<P32, 256><<<grid, 256, 0, st>>>(g, X, Y, red);
-  else redot_kernel<P16, 256><<<grid, 256, 0, st>>>(g, X, Y, red);
-  return launched();
+  if (prec == P64) return launch_chained<P64>(redot_kernel<P64, 256>, grid, 256, 0, st, g, X, Y, red);
+  else if (prec == P32) return launch_chained<P32>(redot_kernel<P32, 256>, grid, 256, 0, st, g, X, Y, red);
+  else return launch_chained<P16>(redot_kernel<P16, 256>, grid, 256, 0, st, g, X, Y, red);
 }
 
 }  // namespace cpsb

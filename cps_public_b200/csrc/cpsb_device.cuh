@@ -130,6 +130,17 @@ struct SpinorPtr {
   long stride;   // entries in the field
 };
 
+// Chained launches of the FP64 kernels (launch_chained): a kernel's blocks may
+// start while the kernel before it in the stream still runs.  Until grid_wait() they
+// touch only what no kernel of a solve or operator writes (links, the lattice
+// geometry); it returns once that kernel and, through its own wait, all before it
+// have finished and their writes are visible.  Every thread of every such kernel calls
+// it.  FP64 fields are therefore read with plain loads: the read-only path (__ldg)
+// is for data that does not change while the kernel exists, waiting included.
+// grid_release() lets the next kernel's blocks start where this one leaves room.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 template <int P> struct PrecTraits;
 template <> struct PrecTraits<P64> { typedef double real; };
 template <> struct PrecTraits<P32> { typedef float real; };
@@ -174,7 +185,7 @@ __device__ __forceinline__ Spinor<double> load_spinor<P64>(const SpinorPtr &f, l
   Spinor<double> s;
 #pragma unroll
   for (int k = 0; k < 12; k++) {
-    double2 v = __ldg(b + 8 * k);
+    const double2 v = b[8 * k];
     s.c[k / 3][k % 3] = mk(v.x, v.y);
   }
   return s;

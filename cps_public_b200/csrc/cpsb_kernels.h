@@ -50,6 +50,34 @@ inline cudaError_t launched() {
   return cudaGetLastError();
 }
 
+// Launches a kernel that calls grid_wait() (P64 ones) so that it may start while the
+// kernel before it in the stream drains (programmatic dependent launch; in a
+// captured graph a programmatic edge): the launch latency, the index tables and the
+// first links' loads of a hop pass behind the tail of its predecessor.  FP64 CG, DWF
+// 8^4, Ls 16: 8.44 -> 7.69 ms; 16^3x32, Ls 16: 323 -> 315 ms; 12-shift MInvCG, Ls 12: 244
+// -> 237 ms; FmatInv 8^3x16, Ls 8 (its FP64 residuals): 12.4 -> 12.0 ms.
+// FP32 and 16-bit kernels are launched plainly: without the read-only path for their
+// fields the same solves got slower (Wilson 24^3x64 FP32 40.1 -> 40.9 ms, DWF 12^3x24,
+// Ls 10, 3 right-hand sides 76.5 -> 77.6 ms).
+template <int P, class... K, class... T>
+cudaError_t launch_chained(void (*kernel)(K...), dim3 grid, unsigned nt, size_t shm, cudaStream_t st, const T &...args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = dim3(nt);
+  c.dynamicSmemBytes = shm;
+  c.stream = st;
+  if (P == P64) {
+    c.attrs = &at;
+    c.numAttrs = 1;
+  }
+  const cudaError_t e = cudaLaunchKernelEx(&c, kernel, static_cast<K>(args)...);
+  if (e != cudaSuccess) return e;
+  return launched();
+}
+
 // Grid: blockIdx.y = right-hand side, blockIdx.x strides over the sites of one RHS.
 int grid_blocks(long sites_per_rhs, int nt);
 

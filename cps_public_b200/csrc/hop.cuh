@@ -114,7 +114,7 @@ template <> __device__ __forceinline__ Raw<P64> load_raw<P64>(const SpinorPtr &f
   const double2 *b = entry_ptr<12, double2>(f.data, i);
   Raw<P64> r;
 #pragma unroll
-  for (int k = 0; k < 12; k++) r.c[k] = __ldg(b + 8 * k);
+  for (int k = 0; k < 12; k++) r.c[k] = b[8 * k];
   return r;
 }
 // The same through L2 only (ld.global.cg): for kernels that read a field that
@@ -600,8 +600,8 @@ __device__ __forceinline__ Spinor<double> hop_entry_64(const DslashArgs &A, cons
     double2 vm[6], vp[6];
 #pragma unroll
     for (int q = 0; q < 6; q++) {
-      vm[q] = L2ONLY ? __ldcg(bm + 8 * (um + q)) : __ldg(bm + 8 * (um + q));
-      vp[q] = L2ONLY ? __ldcg(bp + 8 * (up + q)) : __ldg(bp + 8 * (up + q));
+      vm[q] = L2ONLY ? __ldcg(bm + 8 * (um + q)) : bm[8 * (um + q)];
+      vp[q] = L2ONLY ? __ldcg(bp + 8 * (up + q)) : bp[8 * (up + q)];
     }
 #pragma unroll
     for (int q = 0; q < 6; q++) {
@@ -887,13 +887,7 @@ __global__ void __launch_bounds__(NT, MINB) hop_kernel(DslashArgs A) {
   const Geom &g = A.g;
   extern __shared__ __align__(16) unsigned char dsh[];
   __shared__ double red[NT / 32];
-  // alpha = |r|^2 / (<p, A p> + shift |p|^2) per right-hand side, once per block
-  // (the loop over units starts with a barrier)
   __shared__ double cg_alpha[MAX_RHS];
-  if (CGR && threadIdx.x < g.nrhs) {
-    const CgState *S = A.cg;
-    cg_alpha[threadIdx.x] = S->rr[threadIdx.x] / (S->d[threadIdx.x] + S->shift * S->pp[threadIdx.x]);
-  }
   const int C0 = g.cs[0];
   const int TX = NT / C0;
   const HopShm L = hop_shm(TX, NT, g.nrhs, NORM || CGR, LC);
@@ -906,11 +900,24 @@ __global__ void __launch_bounds__(NT, MINB) hop_kernel(DslashArgs A) {
   const int ncls = g.ncls;
   const int nunits = ntiles * ncls;
   const unsigned per = (unsigned)g.n4cb * (unsigned)g.ls;
-  for (int unit = blockIdx.x; unit < nunits; unit += gridDim.x) {
+  for (int unit = blockIdx.x;; unit += gridDim.x) {
     const int k = unit % ncls, tile = tile_order(g, unit / ncls, TX, A.torder);
     const int par_out = A.five_d ? ((1 - A.cb + k) & 1) : 1 - A.cb;
-    __syncthreads();  // the previous unit is done with the tables
-    load_unit<P, LC>(A, tile, k, par_out, TX, NT, dsh);
+    const bool first = unit == (int)blockIdx.x;
+    if (!first) __syncthreads();  // the previous unit is done with the tables
+    if (unit < nunits) load_unit<P, LC>(A, tile, k, par_out, TX, NT, dsh);
+    if (first) {
+      if (P == P64) {  // the first unit's tables are made while the kernel before drains
+        grid_wait();
+        grid_release();
+      }
+      // alpha = |r|^2 / (<p, A p> + shift |p|^2) per right-hand side, once per block
+      if (CGR && threadIdx.x < g.nrhs) {
+        const CgState *S = A.cg;
+        cg_alpha[threadIdx.x] = S->rr[threadIdx.x] / (S->d[threadIdx.x] + S->shift * S->pp[threadIdx.x]);
+      }
+    }
+    if (unit >= nunits) break;
     __syncthreads();
     const int x = tile * TX + xl;
     const int C = g.cs[k];
@@ -1030,6 +1037,8 @@ __global__ void __launch_bounds__(NT) hop8_kernel(DslashArgs A) {
   __shared__ double cg_alpha[MAX_RHS];
   double2 *gsh = (double2 *)dsh;                        // 12 x NT partial-spinor slots
   double *nrm_sh = (double *)(dsh + (size_t)12 * NT * sizeof(double2));
+  grid_wait();
+  grid_release();
   if (CGR && threadIdx.x < g.nrhs) {
     const CgState *S = A.cg;
     cg_alpha[threadIdx.x] = S->rr[threadIdx.x] / (S->d[threadIdx.x] + S->shift * S->pp[threadIdx.x]);
@@ -1085,7 +1094,7 @@ __global__ void __launch_bounds__(NT) hop8_kernel(DslashArgs A) {
         const int chunk0 = (d == 0) != DAG ? 0 : 6;
         const double2 *b = entry_ptr<12, const double2>(A.in.data, rb + site_entry(g, sn, x));
 #pragma unroll
-        for (int qq = 0; qq < 6; qq++) v5[qq] = __ldg(b + 8 * (chunk0 + qq));
+        for (int qq = 0; qq < 6; qq++) v5[qq] = b[8 * (chunk0 + qq)];
         f5m = s == 0 ? A.hop5_wall : A.hop5_fact;
         f5p = s == g.ls - 1 ? A.hop5_wall : A.hop5_fact;
       }
@@ -1246,7 +1255,7 @@ static cudaError_t hop_launch_v(DslashArgs A, int xpay, int norm, cudaStream_t s
     e = opt_in(fn, done);                                                                  \
     if (e != cudaSuccess) return e;                                                        \
     const long nb = std::min(units, (long)resident_blocks(fn, NT, L.total));                \
-    hop_kernel<P, NT, MINB, LC, XP, NR, CG, D, DEPTH, CROSS><<<(unsigned)nb, NT, L.total, st>>>(A);      \
+    return launch_chained<P>(hop_kernel<P, NT, MINB, LC, XP, NR, CG, D, DEPTH, CROSS>, dim3((unsigned)nb), NT, L.total, st, A); \
   }
 #define CPSB_HOP_D(XP, NR, CG)          \
   if (A.dag) CPSB_HOP(XP, NR, CG, true) \
@@ -1259,7 +1268,6 @@ static cudaError_t hop_launch_v(DslashArgs A, int xpay, int norm, cudaStream_t s
   else CPSB_HOP_D(false, false, 0)
 #undef CPSB_HOP_D
 #undef CPSB_HOP
-  return launched();
 }
 
 // The direction-parallel FP64 hop: eight lanes per entry, the grid no larger
@@ -1275,7 +1283,7 @@ static cudaError_t hop8_launch(const DslashArgs &A, int xpay, int norm, cudaStre
   {                                                                                \
     const void *fn = (const void *)hop8_kernel<NT, XP, NR, CG, D>;                 \
     const long nb = std::min(want, (long)resident_blocks(fn, NT, shm));            \
-    hop8_kernel<NT, XP, NR, CG, D><<<(unsigned)nb, NT, shm, st>>>(A);              \
+    return launch_chained<P64>(hop8_kernel<NT, XP, NR, CG, D>, dim3((unsigned)nb), NT, shm, st, A); \
   }
 #define CPSB_HOP8_D(XP, NR, CG)          \
   if (A.dag) CPSB_HOP8(XP, NR, CG, true) \
@@ -1288,7 +1296,6 @@ static cudaError_t hop8_launch(const DslashArgs &A, int xpay, int norm, cudaStre
   else CPSB_HOP8_D(false, false, 0)
 #undef CPSB_HOP8_D
 #undef CPSB_HOP8
-  return launched();
 }
 
 // Launch shapes the autotuner chooses from.  Shapes with link tables need columns of

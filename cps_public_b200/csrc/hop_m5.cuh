@@ -44,10 +44,6 @@ __global__ void __launch_bounds__(NT, MINB) hop_m5_kernel(DslashArgs A, M5Coef c
   extern __shared__ __align__(16) unsigned char dsh[];
   __shared__ double red[NT / 32];
   __shared__ double cg_alpha[MAX_RHS];  // as in hop_kernel
-  if (CGR && threadIdx.x < g.nrhs) {
-    const CgState *S = A.cg;
-    cg_alpha[threadIdx.x] = S->rr[threadIdx.x] / (S->d[threadIdx.x] + S->shift * S->pp[threadIdx.x]);
-  }
   const HopShm L = hop_shm(TX, NT, g.nrhs, NORM || CGR, true);
   BT *tile_buf = (BT *)(dsh + hop_m5_tile_off<P, LS>(TX, NT, g.nrhs, NORM || CGR));
   double *nrm_sh = (double *)(dsh + L.norm);
@@ -58,9 +54,20 @@ __global__ void __launch_bounds__(NT, MINB) hop_m5_kernel(DslashArgs A, M5Coef c
   const int ntiles = (g.n4cb + TX - 1) / TX;
   const unsigned per = (unsigned)g.n4cb * (unsigned)LS;
   const int par_out = 1 - A.cb;
+  if ((int)blockIdx.x < ntiles) load_unit<P, true>(A, blockIdx.x, 0, par_out, TX, NT, dsh);
+  if (P == P64) {  // as in hop_kernel
+    grid_wait();
+    grid_release();
+  }
+  if (CGR && threadIdx.x < g.nrhs) {
+    const CgState *S = A.cg;
+    cg_alpha[threadIdx.x] = S->rr[threadIdx.x] / (S->d[threadIdx.x] + S->shift * S->pp[threadIdx.x]);
+  }
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    __syncthreads();  // the previous tile is done with the tables and the sweep tile
-    load_unit<P, true>(A, tile, 0, par_out, TX, NT, dsh);
+    if (tile != (int)blockIdx.x) {
+      __syncthreads();  // the previous tile is done with the tables and the sweep tile
+      load_unit<P, true>(A, tile, 0, par_out, TX, NT, dsh);
+    }
     __syncthreads();
     const int x = tile * TX + xl;
     const bool act = xl < TX && x < g.n4cb;
@@ -169,8 +176,7 @@ static cudaError_t hop_m5_launch_m(const DslashArgs &A, const M5Coef &cf, cudaSt
   }
   const long ntiles = (A.g.n4cb + TX - 1) / TX;
   const long nb = std::min(ntiles, (long)resident_blocks(fn, NT, shm));
-  hop_m5_kernel<P, NT, MINB, DAG, XPAY, NORM, CGR, LS, DEPTH><<<(unsigned)nb, NT, shm, st>>>(A, cf);
-  return launched();
+  return launch_chained<P>(hop_m5_kernel<P, NT, MINB, DAG, XPAY, NORM, CGR, LS, DEPTH>, dim3((unsigned)nb), NT, shm, st, A, cf);
 }
 
 template <int P, int LS>

@@ -136,6 +136,10 @@ __global__ void __launch_bounds__(NT) ms_r_update_kernel(Geom g, SpinorPtr rout,
                                                          SpinorPtr p0, MsBatch *B, int slot, Reduce red) {
   typedef typename PrecTraits<P>::real T;
   __shared__ double sh[NT / 32];
+  if (P == P64) {
+    grid_wait();
+    grid_release();
+  }
   const int q = blockIdx.y;
   const MsState *S = &B->s[q];
   const long n = (long)g.n4cb * g.ls;
@@ -193,6 +197,10 @@ __global__ void __launch_bounds__(NT) ms_xp_update_kernel(Geom g, SpinorPtr r, S
   typedef typename PrecTraits<P>::real T;
   typedef typename PrecTraits<PX>::real TX;
   __shared__ double sh[NT / 32];
+  if (P == P64) {
+    grid_wait();
+    grid_release();
+  }
   const int q = blockIdx.y;
   const MsState *S = &B->s[q];
   const long n = (long)g.n4cb * g.ls;
@@ -303,6 +311,10 @@ __global__ void __launch_bounds__(NT) ms_shift_update_kernel(Geom g, MsGroup R, 
   constexpr int NCH = P == P64 ? 12 : 6;
   __shared__ T f[MAX_SHIFT][MS_GROUP], z[MAX_SHIFT][MS_GROUP], as[MAX_SHIFT][MS_GROUP];
   __shared__ unsigned xm[MS_GROUP], pm[MS_GROUP];
+  if (P == P64) {
+    grid_wait();
+    grid_release();
+  }
   const int q = blockIdx.y;
   const MsState *S = &B->s[q];
   const int ns = S->nshift;
@@ -373,29 +385,26 @@ static int ms_blocks(long n) {
 cudaError_t launch_ms_r_update(int prec, const Geom &g, SpinorPtr rout, SpinorPtr rin, SpinorPtr Ap, SpinorPtr p0,
                                MsBatch *B, int slot, Reduce red, cudaStream_t st) {
   const dim3 grid(ms_blocks((long)g.n4cb * g.ls), g.nrhs);
-  if (prec == P64) ms_r_update_kernel<P64, 256><<<grid, 256, 0, st>>>(g, rout, rin, Ap, p0, B, slot, red);
-  else if (prec == P32) ms_r_update_kernel<P32, 256><<<grid, 256, 0, st>>>(g, rout, rin, Ap, p0, B, slot, red);
-  else ms_r_update_kernel<P16, 256><<<grid, 256, 0, st>>>(g, rout, rin, Ap, p0, B, slot, red);
-  return launched();
+  if (prec == P64) return launch_chained<P64>(ms_r_update_kernel<P64, 256>, grid, 256, 0, st, g, rout, rin, Ap, p0, B, slot, red);
+  else if (prec == P32) return launch_chained<P32>(ms_r_update_kernel<P32, 256>, grid, 256, 0, st, g, rout, rin, Ap, p0, B, slot, red);
+  else return launch_chained<P16>(ms_r_update_kernel<P16, 256>, grid, 256, 0, st, g, rout, rin, Ap, p0, B, slot, red);
 }
 
 cudaError_t launch_ms_xp_update(int prec, int px, const Geom &g, SpinorPtr r, const ShiftPtrs &p, const ShiftPtrs &psi,
                                 MsBatch *B, int upto, Reduce red, cudaStream_t st) {
   const dim3 grid(ms_blocks((long)g.n4cb * g.ls), g.nrhs);
-  if (prec == P64 && px == P64) ms_xp_update_kernel<P64, P64, 256><<<grid, 256, 0, st>>>(g, r, p, psi, B, upto, red);
-  else if (prec == P32 && px == P32) ms_xp_update_kernel<P32, P32, 256><<<grid, 256, 0, st>>>(g, r, p, psi, B, upto, red);
-  else if (prec == P16 && px == P32) ms_xp_update_kernel<P16, P32, 256><<<grid, 256, 0, st>>>(g, r, p, psi, B, upto, red);
-  else return cudaErrorInvalidValue;
-  return launched();
+  if (prec == P64 && px == P64) return launch_chained<P64>(ms_xp_update_kernel<P64, P64, 256>, grid, 256, 0, st, g, r, p, psi, B, upto, red);
+  else if (prec == P32 && px == P32) return launch_chained<P32>(ms_xp_update_kernel<P32, P32, 256>, grid, 256, 0, st, g, r, p, psi, B, upto, red);
+  else if (prec == P16 && px == P32) return launch_chained<P16>(ms_xp_update_kernel<P16, P32, 256>, grid, 256, 0, st, g, r, p, psi, B, upto, red);
+  return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_ms_shift_update(int prec, const Geom &g, const MsGroup &R, const ShiftPtrs &p, const ShiftPtrs &psi,
                                    const MsBatch *B, int count, cudaStream_t st) {
   const dim3 grid(ms_blocks((long)g.n4cb * g.ls), g.nrhs);
-  if (prec == P64) ms_shift_update_kernel<P64, 256><<<grid, 256, 0, st>>>(g, R, p, psi, B, count);
-  else if (prec == P32) ms_shift_update_kernel<P32, 256><<<grid, 256, 0, st>>>(g, R, p, psi, B, count);
-  else return cudaErrorInvalidValue;
-  return launched();
+  if (prec == P64) return launch_chained<P64>(ms_shift_update_kernel<P64, 256>, grid, 256, 0, st, g, R, p, psi, B, count);
+  else if (prec == P32) return launch_chained<P32>(ms_shift_update_kernel<P32, 256>, grid, 256, 0, st, g, R, p, psi, B, count);
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace cpsb
