@@ -274,10 +274,15 @@ cudaError_t launch_ms_loop_cond(cudaGraphConditionalHandle h, const MsBatch *B, 
 CgSolver *get_solver(Gauge *G, const cpsb_dirac_params &p, int sloppy, int nrhs);
 
 // The persistent FP64 CG loop (cg_persistent.cu).  CPSB_PERSISTENT_CG in the
-// environment: 0 off, 1 (default) for Wilson fields of at most PCG_AUTO_SITES
-// entries (its direction-parallel form, faster than the graph loop there), 2
-// for any action and any size that fits one cooperative launch.
-constexpr long PCG_AUTO_SITES = 1L << 14;
+// environment: 0 off, 1 (default) for Wilson fields of at most PCG_AUTO_SITES entries
+// and DWF ones of half that (its direction-parallel form), 2 for any size that fits
+// one cooperative launch.  The line lies where the resident blocks cover the field
+// in one round (2 blocks of 16 entries an SM); DWF slices share links that this form
+// loads for each.  A solve from host arrays by this loop and by the graph loop:
+// Wilson 8^4 (2048 entries) 1.51 and 2.29 ms, 8^3x16 (4096) 2.49 and 2.91, 12^3x16
+// (13824) 5.58 and 3.72; DWF 4^4, Ls 8 (1024) 4.70 and 6.11 ms, 4^3x8, Ls 16 (4096)
+// 8.58 and 8.45, 6^4, Ls 16 (10368) 14.0 and 7.1.
+constexpr long PCG_AUTO_SITES = 1L << 12;
 constexpr size_t PCG_PARTIAL_SLOTS = (size_t)MAX_RHS * 148 * 16;
 int persistent_cg_mode();
 cudaError_t launch_persistent_cg(const DslashArgs &base, double mkappa2, SpinorPtr t1, SpinorPtr t2, SpinorPtr r,
