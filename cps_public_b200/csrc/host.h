@@ -69,6 +69,8 @@ struct NoCallPool {
   bool was_on;
 };
 void trim_pool();  // returns the memory that the pool keeps unused to the device
+// Whether `bytes` are free on the device, after a trim of the pool if need be.
+bool room_beside_pool(size_t bytes);
 
 // Device allocation that remembers its size; freed on destruction.
 struct DevBuf {
@@ -112,6 +114,10 @@ struct Field {
   Field() = default;
   Field(int prec, long nsites) { create(prec, nsites); }
   void create(int prec, long nsites);
+  void free() {
+    data.alloc(0);
+    norm.alloc(0);
+  }
   SpinorPtr ptr() const { return SpinorPtr{data.p, (float *)norm.p, nsites}; }
   // The entries [off, off + n) of the field as a field of its own: one
   // right-hand side of a multi-RHS field.  off is a multiple of 8 (a whole

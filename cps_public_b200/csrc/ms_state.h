@@ -16,6 +16,10 @@ constexpr int MAX_SHIFT = 32;
 // ms_shift_update_kernel).
 constexpr int MS_GROUP = 4;
 
+// Device memory that the spare residuals of a group leave free (bytes): the
+// instantiated iteration graph and lazily loaded kernels come out of it.
+constexpr size_t MS_SPARE_MARGIN = (size_t)256 << 20;
+
 // What one iteration does to the shifts s >= 1: psi_s -= bs_s p_s for the shifts
 // in x_mask, then p_s = z_s r + as_s p_s for those in p_mask.
 struct MsStep {

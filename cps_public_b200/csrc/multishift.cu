@@ -466,11 +466,18 @@ int multishift_multi(Gauge *G, const cpsb_dirac_params &p, const cpsb_cg_arg &a,
   // iteration, keep one pass over all shifts per iteration.
   const bool grouped = prec != P16 && nshift > 1;
   int group = grouped && spare && ktype == 0 ? (batch < MS_GROUP ? batch : MS_GROUP) : 1;
+  DevBuf state(sizeof(MsBatch)), loopbuf(sizeof(LoopCtl));
+  G->ptr(prec);  // the links that the operator reads, made on their first use
+  // The spare residuals come after everything that the Krylov phase cannot do
+  // without, and go again if they leave the driver no room for the graph; the
+  // refinement gets their memory back (below).
   std::vector<std::unique_ptr<Field>> rf;
+  rf.emplace_back(new Field(prec, n));
   try {
-    for (int j = 0; j < group; j++) rf.emplace_back(new Field(prec, n));
+    while ((int)rf.size() < group) rf.emplace_back(new Field(prec, n));
+    if (group > 1 && !room_beside_pool(MS_SPARE_MARGIN)) throw Error{CPSB_ERR_OOM, "no room beside the spare residuals"};
   } catch (const Error &e) {
-    if (e.code != CPSB_ERR_OOM || rf.empty()) throw;
+    if (e.code != CPSB_ERR_OOM) throw;
     rf.resize(1);
     group = 1;
   }
@@ -520,7 +527,6 @@ int multishift_multi(Gauge *G, const cpsb_dirac_params &p, const cpsb_cg_arg &a,
     any |= !idle;
   }
   const MsBatch init = *hb;
-  DevBuf state(sizeof(MsBatch));
   MsBatch *B = (MsBatch *)state.p;
   CK(cudaMemcpyAsync(state.p, &init, sizeof(MsBatch), cudaMemcpyHostToDevice, st));
   ShiftPtrs pp_, xx_;
@@ -548,7 +554,6 @@ int multishift_multi(Gauge *G, const cpsb_dirac_params &p, const cpsb_cg_arg &a,
     };
     // one graph launch runs batches on the device until every vector is done
     // (graph_loop.cu); else the host replays single batches
-    DevBuf loopbuf(sizeof(LoopCtl));
     LoopCtl *hl = nullptr;
     CK(cudaMallocHost((void **)&hl, 2 * sizeof(LoopCtl)));
     struct LoopPin {
@@ -623,6 +628,12 @@ int multishift_multi(Gauge *G, const cpsb_dirac_params &p, const cpsb_cg_arg &a,
     // Refine every shift with mixed-precision CG on (A + shift_s) to its own
     // tolerance, checked with the FP64 true residual: one solve over all
     // vectors per shift, each vector to its own stop_rsd.
+    // The Krylov phase is over (its stream has been waited for): its vectors make
+    // room for the refinement solver, which a first call allocates here.
+    rf.clear();
+    Ap.free();
+    for (Field &f : pv) f.free();
+    CK(cudaStreamSynchronize(st));
     CgSolver *cg = refiner ? refiner : get_solver(G, p, prec, nvec);
     std::unique_lock<std::mutex> lk(cg->busy, std::defer_lock);
     if (!refiner) lk.lock();  // the cached solver may be shared between threads

@@ -127,6 +127,15 @@ void trim_pool() {
   cudaGetLastError();
 }
 
+bool room_beside_pool(size_t bytes) {
+  size_t fr = 0, tot = 0;
+  CK(cudaMemGetInfo(&fr, &tot));
+  if (fr >= bytes) return true;
+  trim_pool();
+  CK(cudaMemGetInfo(&fr, &tot));
+  return fr >= bytes;
+}
+
 DevBuf::DevBuf(size_t n) { alloc(n); }
 void DevBuf::release() {
   if (!p) return;
