@@ -39,13 +39,12 @@ Context &ctx();
 // Device memory of a call's own buffers.  While a CallPool is alive on a thread,
 // the DevBufs that the thread allocates come from the library's memory pool,
 // ordered on the call's stream: allocated when the stream gets there and given
-// back behind the stream's work, so an early exit needs no synchronisation and
-// calls on other streams and threads never share memory in use.  The pool keeps
+// back behind the stream's work, so calls on other streams and threads never share
+// memory in use; the CallPool waits for the stream when the call ends.  The pool keeps
 // at most an eighth of the device's memory between calls (CUDA returns the rest
-// at the next synchronisation) and gives that back too when the last resident gauge
+// at that wait) and gives that back too when the last resident gauge
 // field is freed, when an allocation fails and before free memory is reported
-// (trim_pool).  Buffers that
-// outlive the call (solvers, gauge copies, staging) are allocated under a
+// (trim_pool).  Buffers that outlive the call (solvers, gauge copies, staging) are allocated under a
 // NoCallPool, with cudaMalloc.  Without the pool every operator call paid
 // cudaMalloc and cudaFree of each of its vectors: 4-8 ms of a 13 ms MatPcDagMatPc
 // (16^3x32, Ls 16, 12 right-hand sides, 16-bit), 270 of 590 ms of a 12-shift MInvCG.

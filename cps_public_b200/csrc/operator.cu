@@ -108,7 +108,12 @@ CallPool::CallPool(cudaStream_t st) : was_on(t_pool_on), was(t_pool_stream) {
     }
   }
 }
+// The frees of the call's buffers are in the stream by now.  CUDA gives their memory
+// to the device (trim_pool, the bound on what the pool keeps) only once the host has
+// seen them pass: the 3.2 GB of a 16^3x16, Ls 16, 8-source MatPcDagMatPc otherwise
+// stay with the pool whatever is trimmed.
 CallPool::~CallPool() {
+  if (t_pool_on && cudaStreamSynchronize(t_pool_stream) != cudaSuccess) cudaGetLastError();
   t_pool_on = was_on;
   t_pool_stream = was;
 }

@@ -71,3 +71,50 @@ def test_refused_call_leaves_the_pool_usable():
     with pytest.raises(cb.CpsbError):
         bad.MatPc(np.zeros(bad.n))
     assert np.array_equal(_mdagm(op, b, cb.F64), want)
+
+
+def _small(cb):
+    """Loads every kernel of the large calls below."""
+    cb, op, b = _setup((8, 8, 8, 8), 16, 8)
+    _mdagm(op, b, cb.F64)
+
+
+def test_memory_of_a_large_call_is_given_back():
+    """Free memory as reported right after a call of 3.2 GB of vectors is what it was before the call."""
+    import torch
+    cb, op, b = _setup((16, 16, 16, 16), 16, 8)
+    _small(cb)
+    out = torch.empty_like(b)
+    del out  # stays with torch, for the result of the call
+    free0, _ = cb.mem_info()
+    _mdagm(op, b, cb.F64)
+    free1, _ = cb.mem_info()
+    assert free0 - free1 < 64 << 20, (free0, free1)
+
+
+LAST_GAUGE = """
+import torch
+from tests.test_gpu_call_pool import _mdagm, _setup, _small
+cb, op, b = _setup((16, 16, 16, 16), 16, 8)
+_small(cb)
+out = torch.empty_like(b)
+del out  # stays with torch, for the result of the call
+cb.mem_info()
+free0 = torch.cuda.mem_get_info()[0]
+_mdagm(op, b, cb.F64)
+kept = free0 - torch.cuda.mem_get_info()[0]
+op.gauge.free()
+freed = torch.cuda.mem_get_info()[0]
+assert kept > 2 << 30, kept         # what the pool keeps between calls
+assert free0 - freed < 64 << 20, (free0, freed)
+"""
+
+
+def test_last_gauge_gives_the_pool_back():
+    """A process of its own: no other gauge field may be resident."""
+    import pathlib
+    import subprocess
+    import sys
+    root = pathlib.Path(__file__).resolve().parents[1]
+    r = subprocess.run([sys.executable, "-c", LAST_GAUGE], cwd=root, capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stderr[-2000:]
