@@ -44,8 +44,8 @@ Context &ctx();
 // at most an eighth of the device's memory between calls (CUDA returns the rest
 // at that wait) and gives that back too when the last resident gauge
 // field is freed, when an allocation fails and before free memory is reported
-// (trim_pool).  Buffers that outlive the call (solvers, gauge copies, staging) are allocated under a
-// NoCallPool, with cudaMalloc.  Without the pool every operator call paid
+// (trim_pool).  Buffers that outlive the call (solvers, gauge copies, staging) are
+// allocated under a NoCallPool, with cudaMalloc.  Without the pool every operator call paid
 // cudaMalloc and cudaFree of each of its vectors: 4-8 ms of a 13 ms MatPcDagMatPc
 // (16^3x32, Ls 16, 12 right-hand sides, 16-bit), 270 of 590 ms of a 12-shift MInvCG.
 struct CallPool {
@@ -63,9 +63,6 @@ struct NoCallPool {
   ~NoCallPool();
   NoCallPool(const NoCallPool &) = delete;
   NoCallPool &operator=(const NoCallPool &) = delete;
-
- private:
-  bool was_on;
 };
 void trim_pool();  // returns the memory that the pool keeps unused to the device
 // Whether `bytes` are free on the device, after a trim of the pool if need be.

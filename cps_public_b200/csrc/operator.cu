@@ -48,7 +48,8 @@ Context &ctx() {
 
 // ----------------------------------------------------------------- memory
 namespace {
-thread_local bool t_pool_on = false;
+thread_local bool t_pool_on = false;    // a CallPool is alive: a call on t_pool_stream
+thread_local int t_no_pool = 0;         // NoCallPools alive
 thread_local cudaStream_t t_pool_stream = nullptr;
 std::mutex pool_mu;
 std::map<int, cudaMemPool_t> &pools() {  // one per device, kept until exit
@@ -117,8 +118,8 @@ CallPool::~CallPool() {
   t_pool_on = was_on;
   t_pool_stream = was;
 }
-NoCallPool::NoCallPool() : was_on(t_pool_on) { t_pool_on = false; }
-NoCallPool::~NoCallPool() { t_pool_on = was_on; }
+NoCallPool::NoCallPool() { t_no_pool++; }
+NoCallPool::~NoCallPool() { t_no_pool--; }
 
 void trim_pool() {
   int dev = 0;
@@ -153,7 +154,7 @@ void DevBuf::alloc(size_t n) {
   release();
   if (n == 0) return;
   pooled = false;
-  if (t_pool_on) {
+  if (t_pool_on && !t_no_pool) {
     if (cudaMemPool_t pool = call_pool()) {
       const cudaError_t e = cudaMallocFromPoolAsync(&p, n, pool, t_pool_stream);
       if (e == cudaSuccess) {
@@ -169,10 +170,13 @@ void DevBuf::alloc(size_t n) {
   }
   cudaError_t e = cudaMalloc(&p, n);
   if (e == cudaErrorMemoryAllocation) {
-    // what the pool keeps, freed once the work behind it is done
+    // What the pool keeps: finished calls have seen their frees pass, this one waits
+    // for its own.  Not for the device: another thread may be recording a graph on
+    // its stream, during which CUDA bars a wait for all streams, or may have long
+    // work queued.
     cudaGetLastError();
     p = nullptr;
-    cudaDeviceSynchronize();
+    if (t_pool_on && cudaStreamSynchronize(t_pool_stream) != cudaSuccess) cudaGetLastError();
     trim_pool();
     e = cudaMalloc(&p, n);
   }

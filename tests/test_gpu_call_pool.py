@@ -118,3 +118,40 @@ def test_last_gauge_gives_the_pool_back():
     root = pathlib.Path(__file__).resolve().parents[1]
     r = subprocess.run([sys.executable, "-c", LAST_GAUGE], cwd=root, capture_output=True, text=True, timeout=600)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_request_loop_beside_refused_calls():
+    """Requests, each of which records its own graph, while another thread's calls are refused for lack of memory."""
+    import torch
+    from cps_public_b200 import _lib, fields
+    cb, opb, b = _setup((16, 16, 16, 16), 16, 8)
+    g = cb.Gauge(fields.random_gauge((4, 4, 4, 4), 0.2, 83), (4, 4, 4, 4))
+    op = cb.DiracOp(g, "dwf", mass=0.1, ls=4)
+    src = fields.random_source(op.n // 24, 84)
+    lib, out = _lib.load(), torch.empty_like(b)
+    free, _ = cb.mem_info()
+    ballast = torch.empty(free - (1 << 30), dtype=torch.uint8, device="cuda")
+    stop, codes = threading.Event(), []
+
+    def refused():
+        while not stop.is_set():
+            codes.append(lib.cpsb_mdagm_multi_dev(opb.gauge.h, C.byref(opb.p), cb.F64, b.shape[0],
+                                                  C.c_void_p(out.data_ptr()), C.c_void_p(b.data_ptr()), None, None))
+
+    th = threading.Thread(target=refused)
+    srv = cb.Server(slots=3, hbm_bytes=400 << 20)
+    th.start()
+    try:
+        first = {}
+        for _ in range(15):
+            ids = [(p, srv.submit(op, [src], stop_rsd=1e-8, precision=p)) for p in (cb.F32, cb.F16, cb.F32)]
+            for p, i in ids:
+                xs = srv.wait(i)[0]
+                assert np.array_equal(first.setdefault(p, xs[0]), xs[0])
+    finally:
+        stop.set()
+        th.join()
+        srv.close()
+        del ballast
+        torch.cuda.empty_cache()
+    assert set(codes) == {-3}  # out of memory, nothing else
