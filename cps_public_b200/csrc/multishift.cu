@@ -186,6 +186,15 @@ __global__ void __launch_bounds__(NT) ms_r_update_kernel(Geom g, SpinorPtr rout,
   }
 }
 
+// a x + y and a x + b y with the roundings spelled out: the one-pass update and the
+// grouped one are different kernels and give the same bits.
+__device__ __forceinline__ double ms_axpy(double a, double x, double y) { return __fma_rn(a, x, y); }
+__device__ __forceinline__ float ms_axpy(float a, float x, float y) { return __fmaf_rn(a, x, y); }
+__device__ __forceinline__ double ms_lin(double a, double x, double b, double y) {
+  return __fma_rn(a, x, __dmul_rn(b, y));
+}
+__device__ __forceinline__ float ms_lin(float a, float x, float b, float y) { return __fmaf_rn(a, x, __fmul_rn(b, y)); }
+
 // psi_s += -bs_s p_s (shifts not frozen at the start of the iteration), then
 // the next directions p_0 = a p_0 + r, p_s = z_s r + as_s p_s; r read once.  Of the
 // shifts below `upto`: 1 where the others follow per group, else all.  Grid row y
@@ -228,8 +237,8 @@ __global__ void __launch_bounds__(NT) ms_xp_update_kernel(Geom g, SpinorPtr r, S
           for (int a = 0; a < 4; a++)
 #pragma unroll
             for (int c = 0; c < 3; c++) {
-              xv.c[a][c].re = tf * (TX)pv.c[a][c].re + xv.c[a][c].re;
-              xv.c[a][c].im = tf * (TX)pv.c[a][c].im + xv.c[a][c].im;
+              xv.c[a][c].re = ms_axpy(tf, (TX)pv.c[a][c].re, xv.c[a][c].re);
+              xv.c[a][c].im = ms_axpy(tf, (TX)pv.c[a][c].im, xv.c[a][c].im);
             }
           if (single) x0 = xv;
           else store_spinor<PX>(psi.v[s], i, xv);
@@ -246,7 +255,9 @@ __global__ void __launch_bounds__(NT) ms_xp_update_kernel(Geom g, SpinorPtr r, S
 #pragma unroll
             for (int a4 = 0; a4 < 4; a4++)
 #pragma unroll
-              for (int c = 0; c < 3; c++) pv.c[a4][c] = cscale(z, rv.c[a4][c]) + cscale(as, pv.c[a4][c]);
+              for (int c = 0; c < 3; c++)
+                pv.c[a4][c] = mk(ms_lin(z, rv.c[a4][c].re, as, pv.c[a4][c].re),
+                                 ms_lin(z, rv.c[a4][c].im, as, pv.c[a4][c].im));
           }
           store_spinor<P>(p.v[s], i, pv);
           if (s == 0) acc += norm2(rounded<P>(pv));
@@ -276,27 +287,27 @@ __global__ void __launch_bounds__(NT) ms_xp_update_kernel(Geom g, SpinorPtr r, S
 // group.  The operations on an element and their order are those of one pass per
 // iteration, so the grouping does not change a result.  Bound by HBM: 4 vectors per
 // running shift and MS_GROUP residuals per group instead of 4 vectors per shift
-// and one residual per iteration.  DWF 16^3x32, Ls 12, 12 shifts, FP64: 442 us an
-// iteration for all shifts before; now 121 us for shift 0 (5 vectors) and 487 us
-// per group for the others, the 250-iteration solve 304 -> 250 ms.
+// and one residual per iteration.  DWF 16^3x32, Ls 12, 12 shifts, FP64 (vectors of 151
+// MB): with all 11 upper shifts running a group takes 1150 us (48 vectors, 6.3 TB/s);
+// over a solve, whose shifts drop out as they converge, 420 us a group and 131 us an
+// iteration for shift 0 (5 vectors) against 442 us an iteration for all shifts in one
+// pass, the 250-iteration solve 304 -> 250 ms.
 // Every operation acts on single reals and p, r and psi have the same layout
 // (FP64, or FP32 for both), so a thread takes one 16-byte chunk at a time through
 // all shifts, with few registers and every warp access contiguous.
-// SINGLE: the contributions of an iteration are summed over the shifts first
-// (acc[j]), then added to psi.
 template <int P> struct MsChunk { typedef double2 V; typedef double T; };
 template <> struct MsChunk<P32> { typedef float4 V; typedef float T; };
 __device__ __forceinline__ double2 axpy_chunk(double a, double2 x, double2 y) {
-  return make_double2(a * x.x + y.x, a * x.y + y.y);
+  return make_double2(ms_axpy(a, x.x, y.x), ms_axpy(a, x.y, y.y));
 }
 __device__ __forceinline__ float4 axpy_chunk(float a, float4 x, float4 y) {
-  return make_float4(a * x.x + y.x, a * x.y + y.y, a * x.z + y.z, a * x.w + y.w);
+  return make_float4(ms_axpy(a, x.x, y.x), ms_axpy(a, x.y, y.y), ms_axpy(a, x.z, y.z), ms_axpy(a, x.w, y.w));
 }
 __device__ __forceinline__ double2 lin_chunk(double a, double2 x, double b, double2 y) {
-  return make_double2(a * x.x + b * y.x, a * x.y + b * y.y);
+  return make_double2(ms_lin(a, x.x, b, y.x), ms_lin(a, x.y, b, y.y));
 }
 __device__ __forceinline__ float4 lin_chunk(float a, float4 x, float b, float4 y) {
-  return make_float4(a * x.x + b * y.x, a * x.y + b * y.y, a * x.z + b * y.z, a * x.w + b * y.w);
+  return make_float4(ms_lin(a, x.x, b, y.x), ms_lin(a, x.y, b, y.y), ms_lin(a, x.z, b, y.z), ms_lin(a, x.w, b, y.w));
 }
 
 struct MsGroup {
@@ -318,7 +329,6 @@ __global__ void __launch_bounds__(NT) ms_shift_update_kernel(Geom g, MsGroup R, 
   const int q = blockIdx.y;
   const MsState *S = &B->s[q];
   const int ns = S->nshift;
-  const bool single = S->type == 1;
   for (int t = threadIdx.x; t < ns * MS_GROUP; t += NT) {
     const int s = t / MS_GROUP, j = t % MS_GROUP;
     const MsStep &st = S->step[j];
@@ -326,7 +336,7 @@ __global__ void __launch_bounds__(NT) ms_shift_update_kernel(Geom g, MsGroup R, 
       xm[j] = j < count ? st.x_mask : 0u;
       pm[j] = j < count ? st.p_mask : 0u;
     } else if (j < count) {
-      f[s][j] = (T)(single ? -st.bs[s] * S->alpha[s] : -st.bs[s]);
+      f[s][j] = (T)-st.bs[s];
       z[s][j] = (T)st.z[s];
       as[s][j] = (T)st.as[s];
     }
@@ -343,34 +353,21 @@ __global__ void __launch_bounds__(NT) ms_shift_update_kernel(Geom g, MsGroup R, 
   const long n = (long)g.n4cb * g.ls * NCH;
   for (long i = (long)blockIdx.x * NT + threadIdx.x; i < n; i += (long)gridDim.x * NT) {
     const long c = q * n + i;
-    V rv[MS_GROUP], acc[MS_GROUP];
+    V rv[MS_GROUP];
 #pragma unroll
-    for (int j = 0; j < MS_GROUP; j++) {
-      rv[j] = pm[j] ? ((const V *)R.r[j].data)[c] : zero;
-      acc[j] = zero;
-    }
+    for (int j = 0; j < MS_GROUP; j++) rv[j] = pm[j] ? ((const V *)R.r[j].data)[c] : zero;
     for (int s = 1; s < ns; s++) {
       const unsigned bit = 1u << s;
       if (!((all_x | all_p) & bit)) continue;
       V pv = ((const V *)p.v[s].data)[c];
-      V xv = !single && (all_x & bit) ? ((const V *)psi.v[s].data)[c] : zero;
+      V xv = (all_x & bit) ? ((const V *)psi.v[s].data)[c] : zero;
 #pragma unroll
       for (int j = 0; j < MS_GROUP; j++) {
-        if (xm[j] & bit) {
-          if (single) acc[j] = axpy_chunk(f[s][j], pv, acc[j]);
-          else xv = axpy_chunk(f[s][j], pv, xv);
-        }
+        if (xm[j] & bit) xv = axpy_chunk(f[s][j], pv, xv);
         if (pm[j] & bit) pv = lin_chunk(z[s][j], rv[j], as[s][j], pv);
       }
       if (all_p & bit) ((V *)p.v[s].data)[c] = pv;
-      if (!single && (all_x & bit)) ((V *)psi.v[s].data)[c] = xv;
-    }
-    if (single) {
-      V xv = ((const V *)psi.v[0].data)[c];
-#pragma unroll
-      for (int j = 0; j < MS_GROUP; j++)
-        if (xm[j]) xv = axpy_chunk((T)1, acc[j], xv);
-      ((V *)psi.v[0].data)[c] = xv;
+      if (all_x & bit) ((V *)psi.v[s].data)[c] = xv;
     }
   }
 }
@@ -459,13 +456,13 @@ int multishift_multi(Gauge *G, const cpsb_dirac_params &p, const cpsb_cg_arg &a,
   DevBuf dres(sizeof(double) * MAX_RHS);
   const int batch = a.batch > 0 ? a.batch : (graph_loops_enabled() ? 4 : 16);
   // The shifts s >= 1 are updated once per `group` iterations, which keeps the
-  // residuals of the group: with `spare` and room for the vectors, else the group is
-  // one iteration and the residual is updated in place.  SINGLE takes groups of one:
-  // shift 0 and the others add to the same vector, so a longer group would change
-  // the order of the sum.  16-bit Krylov vectors, whose rounding is per entry and
-  // iteration, keep one pass over all shifts per iteration.
-  const bool grouped = prec != P16 && nshift > 1;
-  int group = grouped && spare && ktype == 0 ? (batch < MS_GROUP ? batch : MS_GROUP) : 1;
+  // residuals of the group: with `spare` and room for the vectors.  Else, and for
+  // SINGLE (all shifts add to one vector, in the order of the iterations) and 16-bit
+  // Krylov vectors (their rounding is per entry and iteration), one pass updates all
+  // shifts in every iteration and the residual stays in place: it reads r once, and
+  // in SINGLE moves psi once, where groups of one move both twice (16^3x32, Ls 12, 12
+  // shifts, FP64, to 1e-8: SINGLE 148 ms against 182, MULTI 188 against 205).
+  int group = prec != P16 && nshift > 1 && spare && ktype == 0 ? (batch < MS_GROUP ? batch : MS_GROUP) : 1;
   DevBuf state(sizeof(MsBatch)), loopbuf(sizeof(LoopCtl));
   G->ptr(prec);  // the links that the operator reads, made on their first use
   // The spare residuals come after everything that the Krylov phase cannot do
@@ -547,8 +544,8 @@ int multishift_multi(Gauge *G, const cpsb_dirac_params &p, const cpsb_cg_arg &a,
         const int slot = j % group, prev = (j == 0 ? batch - 1 : j - 1) % group;
         op.mdagm(Ap, pv[0], &rd, skip, st);
         CK(launch_ms_r_update(prec, g, rg.r[slot], rg.r[prev], Ap.ptr(), pv[0].ptr(), B, slot, rr, st));
-        CK(launch_ms_xp_update(prec, px, g, rg.r[slot], pp_, xx_, B, grouped ? 1 : nshift, rp, st));
-        if (grouped && (slot == group - 1 || j == batch - 1))
+        CK(launch_ms_xp_update(prec, px, g, rg.r[slot], pp_, xx_, B, group > 1 ? 1 : nshift, rp, st));
+        if (group > 1 && (slot == group - 1 || j == batch - 1))
           CK(launch_ms_shift_update(prec, g, rg, pp_, xx_, B, slot + 1, st));
       }
     };

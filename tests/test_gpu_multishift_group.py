@@ -80,3 +80,15 @@ def test_one_shift_and_limit_inside_a_group():
         xs = [_solve(cb, op, srcs, SHIFTS, cb.F64, batch, cb.MULTI, max_iter=limit) for batch in (1, 4)]
         assert xs[0][2] == xs[1][2] == 1 and xs[0][1] == xs[1][1]
         assert np.array_equal(xs[0][0], xs[1][0]), limit
+
+
+@pytest.mark.parametrize("action,ls", [("wilson", 1), ("dwf", 5), ("mobius", 4)])
+def test_fp32_groups_agree(action, ls):
+    """FP32 Krylov vectors (16-byte chunks of four reals): groups of every length do the operations of one pass per
+    iteration, so the refinement starts from the same solutions and neither it nor the result may differ."""
+    cb, op, srcs = _op(action, ls)
+    x0, it0, rc = _solve(cb, op, srcs, SHIFTS, cb.F32, 1, cb.MULTI, stop=1e-10)
+    assert rc == 0
+    for batch in (3, 4, 5):
+        x, it, rc = _solve(cb, op, srcs, SHIFTS, cb.F32, batch, cb.MULTI, stop=1e-10)
+        assert rc == 0 and it == it0 and np.array_equal(x, x0), batch
