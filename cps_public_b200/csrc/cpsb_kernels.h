@@ -56,6 +56,14 @@ inline cudaError_t launched() {
 // first links' loads of a hop pass behind the tail of its predecessor.  FP64 CG, DWF
 // 8^4, Ls 16: 8.44 -> 7.69 ms; 16^3x32, Ls 16: 323 -> 315 ms; 12-shift MInvCG, Ls 12: 244
 // -> 237 ms; FmatInv 8^3x16, Ls 8 (its FP64 residuals): 12.4 -> 12.0 ms.
+// The kernels of the Mobius 5th dimension (m5_kernel, hop_m5_kernel) are launched
+// plainly and let no successor start early.  Chained they slow every solve that uses
+// them (16^4, FP64 CG to 1e-8, chained and plain: Ls 8 41.3 and 32.1 ms, four sources
+// 161 and 115, SYM1 51.1 and 43.9, ORIG 54.5 and 46.5; Ls 12 55.7 and 53.8), most
+// likely since an SM that holds blocks of two kernels sets aside shared memory for
+// both, which the hops, whose neighbours sit in L1, miss there: with the largest
+// shared-memory share asked for, chained Ls 12 and 16 lose as Ls 8 does (70 for 56
+// ms, 93 for 72).
 // FP32 and 16-bit kernels are launched plainly: without the read-only path for their
 // fields the same solves got slower (Wilson 24^3x64 FP32 40.1 -> 40.9 ms, DWF 12^3x24,
 // Ls 10, 3 right-hand sides 76.5 -> 77.6 ms).

@@ -55,10 +55,6 @@ __global__ void __launch_bounds__(NT, MINB) hop_m5_kernel(DslashArgs A, M5Coef c
   const unsigned per = (unsigned)g.n4cb * (unsigned)LS;
   const int par_out = 1 - A.cb;
   if ((int)blockIdx.x < ntiles) load_unit<P, true>(A, blockIdx.x, 0, par_out, TX, NT, dsh);
-  if (P == P64) {  // as in hop_kernel
-    grid_wait();
-    grid_release();
-  }
   if (CGR && threadIdx.x < g.nrhs) {
     const CgState *S = A.cg;
     cg_alpha[threadIdx.x] = S->rr[threadIdx.x] / (S->d[threadIdx.x] + S->shift * S->pp[threadIdx.x]);
@@ -176,7 +172,8 @@ static cudaError_t hop_m5_launch_m(const DslashArgs &A, const M5Coef &cf, cudaSt
   }
   const long ntiles = (A.g.n4cb + TX - 1) / TX;
   const long nb = std::min(ntiles, (long)resident_blocks(fn, NT, shm));
-  return launch_chained<P>(hop_m5_kernel<P, NT, MINB, DAG, XPAY, NORM, CGR, LS, DEPTH>, dim3((unsigned)nb), NT, shm, st, A, cf);
+  hop_m5_kernel<P, NT, MINB, DAG, XPAY, NORM, CGR, LS, DEPTH><<<(unsigned)nb, NT, shm, st>>>(A, cf);
+  return launched();
 }
 
 template <int P, int LS>

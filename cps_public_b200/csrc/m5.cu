@@ -157,10 +157,6 @@ __global__ void __launch_bounds__(NT) m5_kernel(Geom g, SpinorPtr out, SpinorPtr
   const int ntiles = (g.n4cb + TX - 1) / TX;
   BT *mine = buf + (size_t)(threadIdx.x / LS) * 12 * CST + threadIdx.x % LS;
   double acc = 0;
-  if (P == P64) {
-    grid_wait();
-    grid_release();
-  }
   const bool sk = skip && skip[rhs];
   for (int tile = blockIdx.x; !sk && tile < ntiles; tile += gridDim.x) {
     const int nx = min(TX, g.n4cb - tile * TX);
@@ -237,7 +233,8 @@ static cudaError_t m5_launch(int dag, const Geom &g, SpinorPtr out, SpinorPtr in
   const dim3 grid(ntiles < 148 * 16 ? ntiles : 148 * 16, g.nrhs);
 #define CPSB_M5(D, XP, NR)                                                                  \
   if (dag == D && !!xpay == XP && !!norm == NR) {                                           \
-    return launch_chained<P>(m5_kernel<P, LS, D, XP, NR, NT>, grid, NT, shm, st, g, out, in, x, cf, red, skip); \
+    m5_kernel<P, LS, D, XP, NR, NT><<<grid, NT, shm, st>>>(g, out, in, x, cf, red, skip);   \
+    return launched();                                                                      \
   }
   CPSB_M5(0, false, false) CPSB_M5(0, true, false) CPSB_M5(0, true, true) CPSB_M5(0, false, true)
   CPSB_M5(1, false, false) CPSB_M5(1, true, false) CPSB_M5(1, true, true) CPSB_M5(1, false, true)
