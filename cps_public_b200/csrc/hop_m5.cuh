@@ -153,12 +153,9 @@ __global__ void __launch_bounds__(NT, MINB) hop_m5_kernel(DslashArgs A, M5Coef c
   if (NORM || CGR) hop_reduce<NT, CGR>(A, nrm_sh, red);
 }
 
-template <int P, int LS, bool DAG, bool XPAY, bool NORM, int CGR>
-static cudaError_t hop_m5_launch_m(const DslashArgs &A, const M5Coef &cf, cudaStream_t st) {
+template <int P, int LS, bool DAG, bool XPAY, bool NORM, int CGR, int MINB>
+static cudaError_t hop_m5_launch_v(const DslashArgs &A, const M5Coef &cf, cudaStream_t st) {
   constexpr int NT = 128;
-  // FP64: 168 registers for 12 warps an SM; with 255 for 8 the hops of 24^3x64, Ls 16 took
-  // 1515, 1375 and 1354 us, now 1330, 1317 and 1310
-  constexpr int MINB = P == P64 ? 3 : 4;
   constexpr int DEPTH = P == P64 ? 1 : 2;
   constexpr int TX = NT / LS;
   const size_t shm = hop_m5_shm<P, LS>(TX, NT, A.g.nrhs, NORM || CGR);
@@ -174,6 +171,26 @@ static cudaError_t hop_m5_launch_m(const DslashArgs &A, const M5Coef &cf, cudaSt
   const long nb = std::min(ntiles, (long)resident_blocks(fn, NT, shm));
   hop_m5_kernel<P, NT, MINB, DAG, XPAY, NORM, CGR, LS, DEPTH><<<(unsigned)nb, NT, shm, st>>>(A, cf);
   return launched();
+}
+
+template <int P, int LS, bool DAG, bool XPAY, bool NORM, int CGR>
+static cudaError_t hop_m5_launch_m(const DslashArgs &A, const M5Coef &cf, cudaStream_t st) {
+  if constexpr (P != P64) {
+    return hop_m5_launch_v<P, LS, DAG, XPAY, NORM, CGR, 4>(A, cf, st);
+  } else {
+    // FP64: 168 registers for 3 blocks an SM (24^3x64, Ls 16: 1330, 1317 and 1310 us the
+    // hops, against 1515, 1375 and 1354 with 255 for 2) where there are tiles for a
+    // third block and room beside its tables.  Not at Ls 4, whose 80 KB a block let two
+    // run, nor on fields that two blocks an SM cover: registers spent on nothing.
+    // CG to 1e-8 with 2 and 3: 16^3x32, Ls 4 23.9 and 27.4 ms; 8^4, Ls 8 (128 tiles)
+    // 4.84 and 5.01, 3 sources 9.1 and 9.7; 8^4, Ls 16 (256) 8.13 and 8.26; 12^3x16, Ls 8
+    // (864) 15.4 and 14.8.
+    if constexpr (LS > 4) {
+      const long ntiles = (A.g.n4cb + 128 / LS - 1) / (128 / LS);
+      if (ntiles > 2 * 148) return hop_m5_launch_v<P, LS, DAG, XPAY, NORM, CGR, 3>(A, cf, st);
+    }
+    return hop_m5_launch_v<P, LS, DAG, XPAY, NORM, CGR, 2>(A, cf, st);
+  }
 }
 
 template <int P, int LS>
