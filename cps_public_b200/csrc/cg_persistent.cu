@@ -10,7 +10,7 @@
 // r -= alpha A p, |r|^2 and x += alpha p fused into the last one, as in the
 // launch-per-step loop), then p = r + beta p, separated by grid barriers.
 // Every block keeps its own copy of the recurrence scalars (CgState) in shared
-// memory and sums the per-block partials of each reduction in block order, so
+// memory and sums the per-block partials of each reduction in the same order, so
 // all blocks hold identical scalars and take the same branches; block 0
 // writes the state back when the loop ends.  Fields written inside the launch
 // are read through L2 (ld.global.cg), never through the read-only cache.
@@ -20,10 +20,10 @@
 // next iteration's first two hops, so an iteration is four hops and four grid
 // barriers; it beats the device-side graph loop of solver.cu there and is the default
 // (figures at PCG_AUTO_SITES, host.h).  Larger fields run the column hop of
-// hop_kernel plus a p-update phase (five barriers), no faster than the graph loop
-// (DWF 8^4, Ls 16: 8.7 against 8.5 ms per solve), only when asked for.
+// hop_kernel plus a p-update phase (five barriers), slower than the graph loop
+// (Wilson 8^2x10x16: 4.0 against 2.7 ms per solve), only when asked for.
 //
-// Grid barriers spin on a generation counter with a time limit: a wait that
+// Grid barriers spin on an arrival counter with a time limit: a wait that
 // runs out sets the error flag, every other block leaves at its next wait, and
 // the host reports the error.  The cooperative launch keeps all blocks
 // resident, so the barriers complete in normal operation.
@@ -39,7 +39,7 @@ namespace cpsb {
 // still spreads over many SMs.
 constexpr int PCG_NT_MAX = 128;
 // Fields (all right-hand sides) of at most this many entries use the
-// direction-parallel hop phases (the same bound as the automatic mode).
+// direction-parallel hop phases (the largest bound of the automatic mode).
 constexpr long PCG_DP_SITES = PCG_AUTO_SITES;
 // Longest barrier wait before it gives up (ns of the global timer): far above a
 // phase of any lattice the loop takes, and above kernels of other streams that
@@ -176,9 +176,8 @@ __device__ __forceinline__ void pcg_hop(const DslashArgs &A, const PcgArgs &P, u
 // differ in which chunks and link elements are loaded and in signs, chosen by
 // address or select), the epilogue's operands are loaded before the neighbours, and
 // the lattice indexes of a thread's first entry are made once per launch.
-// Wilson 8^4, mass 0.1, 89 iterations from host arrays: 2.43 -> 1.53 ms a solve (24 ->
-// 14 us an iteration) against one branch per direction, lane 0 alone after the
-// products and a generation barrier.
+// Wilson 8^4, mass 0.1, to 1e-10 from host arrays: 2.43 -> 1.53 ms a solve against one
+// branch per direction, lane 0 alone after the products and a generation barrier.
 // PUPD folds the direction update p = r + beta p of the previous iteration in:
 // MODE 0 forms each neighbour's r + beta p from r and the old p as it loads
 // them, and MODE 1 forms its own entry's, stores it as the new p and uses it as
@@ -247,6 +246,7 @@ __device__ __forceinline__ void pcg8_hop(const DslashArgs &A, const PcgArgs &P, 
     const double b = PUPD ? beta[q] : 0.0;
     for (long e = e_first; e - (threadIdx.x / 8) % 4 < (long)per; e += wstride) {  // all four entries of a warp together
       Pcg8Idx ix = first;
+      // a second round only where fewer than PCG_DP_SITES / 16 blocks are resident
       if (e != e_first) ix = pcg8_index(A, A.cb, e, d);
       const unsigned i = rb + ix.own;
       const bool mine = owner && ix.valid;
@@ -408,9 +408,9 @@ __device__ __forceinline__ void pcg8_hop(const DslashArgs &A, const PcgArgs &P, 
   }
 }
 
-// Per-right-hand-side sums of nrm over the grid, left in out[] of every block:
-// every warp adds the block partials in the same order by itself, so all blocks
-// get the same bits without a further exchange.
+// Per-right-hand-side sums of nrm over the grid, left in out[] of every block: the
+// first warp of each block adds the block partials, a lane every 32nd and then the
+// lanes pairwise, so all blocks get the same bits without a further exchange.
 template <int NT>
 __device__ __forceinline__ bool pcg_reduce(const PcgArgs &P, int nrhs, double *nrm, double *red, double *out,
                                            unsigned &epoch) {
@@ -554,7 +554,6 @@ cudaError_t launch_persistent_cg(const DslashArgs &base, double mkappa2, SpinorP
   const int C0 = g.cs[0];
   if (C0 < 1 || C0 > PCG_NT_MAX) return cudaErrorNotSupported;
   const long per = (long)g.n4cb * g.ls;
-  // eight lanes per entry where even that leaves blocks for every SM to spare
   const bool dp = per * g.nrhs <= PCG_DP_SITES;
   const int nt = dp ? PCG_NT_MAX : C0 == 1 ? 32 : PCG_NT_MAX;
   const int TX = nt / C0;

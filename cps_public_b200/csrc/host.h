@@ -277,13 +277,19 @@ CgSolver *get_solver(Gauge *G, const cpsb_dirac_params &p, int sloppy, int nrhs)
 
 // The persistent FP64 CG loop (cg_persistent.cu).  CPSB_PERSISTENT_CG in the
 // environment: 0 off, 1 (default) for Wilson fields of at most PCG_AUTO_SITES entries
-// and DWF ones of half that (its direction-parallel form), 2 for any size that fits
-// one cooperative launch.  The line lies where the resident blocks cover the field
-// in one round (2 blocks of 16 entries an SM); DWF slices share links that this form
-// loads for each.  A solve from host arrays by this loop and by the graph loop:
-// Wilson 8^4 (2048 entries) 1.51 and 2.29 ms, 8^3x16 (4096) 2.49 and 2.91, 12^3x16
-// (13824) 5.58 and 3.72; DWF 4^4, Ls 8 (1024) 4.70 and 6.11 ms, 4^3x8, Ls 16 (4096)
-// 8.58 and 8.45, 6^4, Ls 16 (10368) 14.0 and 7.1.
+// (all right-hand sides) and DWF ones of half that (its direction-parallel form), 2
+// for any size that fits one cooperative launch.  A block takes 16 entries of one
+// right-hand side after the other, so up to 2368 entries each an SM holds one block:
+// there this loop beats the graph loop by 1.3 to 1.7.  With two blocks an SM Wilson
+// still gains, DWF, whose slices share links that this form loads for each, does not.
+// Several sources gain less than one, but gain, up to the line.  Solve time, graph
+// loop and this one, by entries x sources:
+//   Wilson 128 x1 1.60, 0.95 ms; x8 7.09, 4.81; 512 x4 5.14, 3.85; x8 9.09, 6.96;
+//     1024 x4 5.22, 3.88; 2048 x1 2.13, 1.35; x2 3.22, 2.09; 2560 x1 2.44, 1.98; 4096 x1
+//     2.66, 2.21; 5120 x1 (the other form) 2.73, 3.96
+//   DWF 512 x1 3.52, 2.42; x4 8.49, 6.40; 1024 x2 8.34, 6.63; x4 13.2, 11.7; 2048 x1
+//     5.91, 4.30; x2 8.65, 6.84; 2304 x1 7.39, 5.15; 3072 x1 7.79, 7.23 (Ls 12) and
+//     7.70, 8.16 (Ls 16); 4096 x1 8.44, 8.60
 constexpr long PCG_AUTO_SITES = 1L << 12;
 constexpr size_t PCG_PARTIAL_SLOTS = (size_t)MAX_RHS * 148 * 16;
 int persistent_cg_mode();

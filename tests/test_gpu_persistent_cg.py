@@ -6,10 +6,10 @@ the number of blocks whose partial sums make up each dot product, so their
 iteration counts agree within one and their solutions within 1e-9 relative
 (the bound the FP64 solver keeps against CPS itself).  CPSB_PERSISTENT_CG
 selects the loop: 0 launch-per-step, 1 (default) persistent for Wilson fields
-of at most 2^14 entries, 2 persistent for any action and size.  Fields of at
-most 2^14 entries run eight lanes per entry with the direction update folded
-into the next iteration's hops; larger ones one thread per entry with a
-separate direction-update phase.
+of at most 2^12 entries (all right-hand sides) and DWF ones of at most 2^11, 2
+persistent for Wilson and DWF of any size.  Fields of at most 2^12 entries run
+eight lanes per entry with the direction update folded into the next iteration's
+hops; larger ones one thread per entry with a separate direction-update phase.
 """
 import ctypes as C
 import os
@@ -76,9 +76,9 @@ def test_persistent_wilson_8x8x8x8_config_case():
 
 
 def test_persistent_dwf_multi_rhs_with_zero_source():
-    """DWF 4^3 x 8 x Ls 8, four right-hand sides of different difficulty (one a
-    zero source, halted before the first iteration); right-hand sides halt at
-    different iterations inside the one launch."""
+    """DWF 4^3 x 8 x Ls 8, four right-hand sides of different scale (one a zero
+    source, halted before the first iteration): 8192 entries, the
+    one-thread-per-entry form."""
     import cps_public_b200 as cb
     from cps_public_b200 import fields
     cb.init(0)
@@ -89,7 +89,7 @@ def test_persistent_dwf_multi_rhs_with_zero_source():
             fields.random_source(n, 74)]
     for mass in (0.05, 0.3):
         op = cb.DiracOp(g, "dwf", mass=mass, ls=ls)
-        ra, rb = _compare(op, srcs, mode=2)  # the direction-parallel form with the 5th-direction hop
+        ra, rb = _compare(op, srcs, mode=2)
         assert rb[1].iters == ra[1].iters
 
 
@@ -106,3 +106,33 @@ def test_persistent_forced_at_larger_size():
     n = int(np.prod(dims)) // 2 * ls
     srcs = [fields.random_source(n, 82 + q) for q in range(8)]
     _compare(op, srcs, mode=2)
+
+
+@pytest.mark.parametrize("action,dims,ls,nrhs,mode", [
+    ("wilson", (4, 4, 4, 8), 1, 4, 1),   # 256 entries each
+    ("wilson", (8, 8, 8, 16), 1, 1, 1),  # 4096: the largest by default, two blocks an SM
+    ("dwf", (4, 4, 4, 4), 4, 4, 1),      # 512 each, 2048 in all: the most by default
+    ("dwf", (4, 4, 4, 4), 5, 3, 1),      # classes of three and two slices
+    ("dwf", (4, 4, 4, 8), 11, 1, 2),     # 2816: odd Ls, two blocks on some SMs
+    ("dwf", (4, 4, 4, 4), 8, 4, 2),      # 4096 in all: the largest of the eight-lane form
+    ("dwf", (2, 2, 2, 2), 3, 3, 1),      # 24 each: a last block that is half empty
+])
+def test_eight_lane_form(action, dims, ls, nrhs, mode):
+    """The form with eight lanes per entry over its range: sources that converge at different iterations (powers of
+    the operator on a random one: the more, the fewer low modes) and a zero source among several."""
+    import cps_public_b200 as cb
+    from cps_public_b200 import fields
+    cb.init(0)
+    g = cb.Gauge(fields.random_gauge(dims, 0.2, 91), dims, bc_t=1)
+    op = cb.DiracOp(g, action, mass=0.1, ls=ls)
+    n = int(np.prod(dims)) // 2 * ls
+    srcs = [fields.random_source(n, 92 + q) for q in range(nrhs)]
+    for q in range(1, nrhs):
+        for _ in range(2 * q):
+            srcs[q] = op.MatPcDagMatPc(srcs[q])[0]
+    if nrhs > 2:
+        srcs[1] = np.zeros(n * 24)
+    ra, rb = _compare(op, srcs, mode=mode)
+    if nrhs > 2:
+        assert rb[1].iters == ra[1].iters
+        assert rb[nrhs - 1].iters < rb[0].iters  # they halt apart
