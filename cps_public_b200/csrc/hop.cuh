@@ -44,7 +44,7 @@
 // optionally |out|^2 per right-hand side (NORM), or the CG residual update
 // r -= alpha (D-output + sigma p) with |r|^2 and the recurrence scalars (CGR),
 // where the D output is consumed in registers and not stored, together with
-// the solution update x += alpha p when A.cg_x is set.  Reductions are
+// the solution update x += alpha p.  Reductions are
 // deterministic (partials in block order, summed by the last block).
 #pragma once
 #include <algorithm>
@@ -263,16 +263,15 @@ template <> __device__ __forceinline__ double store_x2<P16>(const SpinorPtr &f, 
 // matrices of project() in cpsb_device.cuh written per spin pair: re[1] is
 // (psi2, psi3) and swp(re[1]) is (psi3, psi2).
 template <int MU> __device__ __forceinline__ HfX2 project_x2(const SpX2 &s, float sg) {
-  constexpr bool SW = false;
   HfX2 h;
 #pragma unroll
   for (int c = 0; c < 3; c++) {
     if (MU == 0) {         // h0 = psi0 + i sg psi3, h1 = psi1 + i sg psi2
-      h.re[c] = fma2(f2b(-sg), SW ? s.im[1][c] : swp(s.im[1][c]), s.re[0][c]);
-      h.im[c] = fma2(f2b(sg), SW ? s.re[1][c] : swp(s.re[1][c]), s.im[0][c]);
+      h.re[c] = fma2(f2b(-sg), swp(s.im[1][c]), s.re[0][c]);
+      h.im[c] = fma2(f2b(sg), swp(s.re[1][c]), s.im[0][c]);
     } else if (MU == 1) {  // h0 = psi0 - sg psi3, h1 = psi1 + sg psi2
-      h.re[c] = fma2(f2(-sg, sg), SW ? s.re[1][c] : swp(s.re[1][c]), s.re[0][c]);
-      h.im[c] = fma2(f2(-sg, sg), SW ? s.im[1][c] : swp(s.im[1][c]), s.im[0][c]);
+      h.re[c] = fma2(f2(-sg, sg), swp(s.re[1][c]), s.re[0][c]);
+      h.im[c] = fma2(f2(-sg, sg), swp(s.im[1][c]), s.im[0][c]);
     } else if (MU == 2) {  // h0 = psi0 + i sg psi2, h1 = psi1 - i sg psi3
       h.re[c] = fma2(f2(-sg, sg), s.im[1][c], s.re[0][c]);
       h.im[c] = fma2(f2(sg, -sg), s.re[1][c], s.im[0][c]);
@@ -1160,32 +1159,7 @@ __global__ void __launch_bounds__(NT) hop8_kernel(DslashArgs A) {
         for (int r = 0; r < 3; r++) acc.c[s2][r] = cscale(a, acc.c[s2][r]);
     }
     if (CGR) {
-      const double alpha = cg_alpha[q];
-      Spinor<double> rv = unpack64(load_raw<P64>(A.cg_r, i));
-      if (CGR == 2 || A.cg_x.data) {
-        const Spinor<double> pv = unpack64(load_raw<P64>(A.cg_p, i));
-        if (CGR == 2) {
-          const double sigma = A.cg->shift;
-#pragma unroll
-          for (int s2 = 0; s2 < 4; s2++)
-#pragma unroll
-            for (int r = 0; r < 3; r++) acc.c[s2][r] = acc.c[s2][r] + cscale(sigma, pv.c[s2][r]);
-        }
-        if (A.cg_x.data) {
-          Spinor<double> xv = unpack64(load_raw<P64>(A.cg_x, i));
-#pragma unroll
-          for (int s2 = 0; s2 < 4; s2++)
-#pragma unroll
-            for (int r = 0; r < 3; r++) xv.c[s2][r] = cscale(alpha, pv.c[s2][r]) + xv.c[s2][r];
-          store_spinor<P64>(A.cg_x, i, xv);
-        }
-      }
-#pragma unroll
-      for (int s2 = 0; s2 < 4; s2++)
-#pragma unroll
-        for (int r = 0; r < 3; r++) rv.c[s2][r] = rv.c[s2][r] - cscale(alpha, acc.c[s2][r]);
-      store_spinor<P64>(A.cg_r, i, rv);
-      nrm_sh[q * NT + threadIdx.x] += norm2(rv);
+      nrm_sh[q * NT + threadIdx.x] += cg_epilogue_64<CGR>(A, i, cg_alpha[q], acc);
     } else {
       store_spinor<P64>(A.out, i, acc);
       if (NORM) nrm_sh[q * NT + threadIdx.x] += norm2(acc);
@@ -1319,9 +1293,9 @@ static cudaError_t hop_launch_p(const DslashArgs &A, int xpay, int norm, int var
     case 7:
       if constexpr (P == P16) return hop_launch_v<P, 256, 2, true, 1, true>(A, xpay, norm, st, 0);
       else return cudaErrorNotSupported;
-    // FP32 and 16-bit without the table: one neighbour and its link ahead (Wilson
-    // 24^3x64, FP32: 70 us against 75 for shape 4)
-    // FP64: eight lanes per entry, one neighbour each (small lattices)
+    // FP64: eight lanes per entry, one neighbour each (small lattices).  FP32 and
+    // 16-bit: without the table, one neighbour and its link ahead (Wilson 24^3x64, FP32:
+    // 70 us against 75 for shape 4).
     case 8:
       if constexpr (P == P64) return hop8_launch<128>(A, xpay, norm, st);
       else return hop_launch_v<P, 128, 4, false, 1>(A, xpay, norm, st, 0);

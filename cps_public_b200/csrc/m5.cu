@@ -16,9 +16,9 @@
 // In the column layout (cpsb_device.cuh) the Ls slices of a 4-D site are
 // consecutive entries, so a block moves a tile of whole columns between HBM
 // and shared memory with coalesced 16-byte accesses (one entry per thread),
-// and the sweeps run from shared memory, one thread per (site, storage chunk)
-// with the column of Ls values in registers: every value is read from HBM and
-// written once.  16-bit storage is decoded on the way in and encoded per site
+// and the sweeps run from shared memory, one thread per (site, complex component)
+// in m5_kernel and per (site, storage chunk) in the zMobius m5t_kernel, with the
+// column of Ls values in registers: every value is read from HBM and written once.  16-bit storage is decoded on the way in and encoded per site
 // (its quantum is the site's maximum) on the way out; the sweep arithmetic is
 // FP32.
 #include <string.h>
@@ -142,8 +142,8 @@ template <int P, int NT> struct M5Tile { static const int TX = NT / ChunkT<P>::N
 // The real-coefficient kernel: out = [x +] scale * v, v the column operations.  A
 // block takes TX = NT / LS whole columns, a thread per entry, through the sweep
 // tile of m5_sweep.cuh, whose rows a warp reads and writes without bank conflicts
-// (whole spinors in shared memory, 192 bytes apart, cost 4 wavefronts for 1).  24^3x64, Ls 16, FP64: 630 -> 420 us (6.5 TB/s);
-// 16^3x32, Ls 12, 16-bit, 4 right-hand sides: 105 -> 73 us.
+// (whole spinors in shared memory, 192 bytes apart, cost 4 wavefronts for 1).
+// 24^3x64, Ls 16, FP64: 630 -> 420 us (6.5 TB/s); 16^3x32, Ls 12, 16-bit, 4 right-hand sides: 105 -> 73 us.
 template <int P, int LS, int DAG, bool XPAY, bool NORM, int NT>
 __global__ void __launch_bounds__(NT) m5_kernel(Geom g, SpinorPtr out, SpinorPtr in, SpinorPtr xv, M5Coef cf,
                                                 Reduce red, const int *skip) {

@@ -129,8 +129,9 @@ __device__ __forceinline__ void ms_advance(MsState *S, double cnew, double d, in
 }
 
 // rout = rin + b (Ap + shift0 p0), b = -c/d; |r|^2; the last block advances the
-// scalars and files the iteration under `slot` of its group.  Grid row y is vector y (entries [y n, (y+1) n)); the rows of
-// finished vectors do no work but take part in the reduction's ticket.
+// scalars and files the iteration under `slot` of its group.  Grid row y is vector y
+// (entries [y n, (y+1) n)); the rows of finished vectors do no work but take part in
+// the reduction's ticket.
 template <int P, int NT>
 __global__ void __launch_bounds__(NT) ms_r_update_kernel(Geom g, SpinorPtr rout, SpinorPtr rin, SpinorPtr Ap,
                                                          SpinorPtr p0, MsBatch *B, int slot, Reduce red) {
