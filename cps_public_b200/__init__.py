@@ -31,6 +31,8 @@ def init(device: int = 0) -> None:
 
 
 def mem_info():
+    """(free, total) device memory in bytes, after giving back what the library keeps between calls (at most an
+    eighth of the device): call it before allocations of the program's own that need that memory."""
     lib = _lib.load()
     f, t = C.c_ulonglong(), C.c_ulonglong()
     check(lib.cpsb_mem_info(C.byref(f), C.byref(t)), "cpsb_mem_info")

@@ -55,7 +55,7 @@ inline cudaError_t launched() {
 // captured graph a programmatic edge): the launch latency, the index tables and the
 // first links' loads of a hop pass behind the tail of its predecessor.  FP64 CG, DWF
 // 8^4, Ls 16: 8.44 -> 7.69 ms; 16^3x32, Ls 16: 323 -> 315 ms; 12-shift MInvCG, Ls 12: 244
-// -> 237 ms; FmatInv 8^3x16, Ls 8 (its FP64 residuals): 12.4 -> 12.0 ms.
+// -> 237 ms.
 // The kernels of the Mobius 5th dimension (m5_kernel, hop_m5_kernel) are launched
 // plainly and let no successor start early.  Chained they slow every solve that uses
 // them (16^4, FP64 CG to 1e-8, chained and plain: Ls 8 41.3 and 32.1 ms, four sources

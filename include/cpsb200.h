@@ -105,6 +105,10 @@ const char *cpsb_error_string(int code);
 /* Detail message of the last error raised on the calling thread. */
 const char *cpsb_last_error(void);
 /* Free and total device memory in bytes (the serving loop admits work by it).
+ * Between calls the library keeps the vectors' memory of the last ones, at most
+ * an eighth of the device, which a host program's own allocations cannot have.
+ * This call gives it back first, as does freeing the last gauge field: a program
+ * that needs the memory itself calls it before it allocates.
  * No counterpart in the reference. */
 int cpsb_mem_info(unsigned long long *free_bytes, unsigned long long *total_bytes);
 
