@@ -93,7 +93,7 @@ bool build_loop_graph(cudaStream_t st, const std::function<void(cudaGraphConditi
   size_t nn = 0;
   CK(cudaGraphGetNodes(body, nullptr, &nn));
   *body_nodes = nn;
-  CK(cudaGraphInstantiate(exec, outer, 0));
+  CK(instantiate_graph(exec, outer));
   return true;
 }
 

@@ -65,8 +65,12 @@ struct NoCallPool {
   NoCallPool &operator=(const NoCallPool &) = delete;
 };
 void trim_pool();  // returns the memory that the pool keeps unused to the device
-// Whether `bytes` are free on the device, after a trim of the pool if need be.
+// Whether `bytes` are free on the device, after a trim of the pool if need be.  Asks
+// the driver, which now and then takes tens of ms to answer: not on every call.
 bool room_beside_pool(size_t bytes);
+size_t pool_reserved();  // device bytes that the pool holds, in use or kept
+// cudaGraphInstantiate; where the device is full, again after a trim of the pool.
+cudaError_t instantiate_graph(cudaGraphExec_t *exec, cudaGraph_t graph);
 
 // Device allocation that remembers its size; freed on destruction.
 struct DevBuf {

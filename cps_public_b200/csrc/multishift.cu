@@ -467,13 +467,15 @@ int multishift_multi(Gauge *G, const cpsb_dirac_params &p, const cpsb_cg_arg &a,
   DevBuf state(sizeof(MsBatch)), loopbuf(sizeof(LoopCtl));
   G->ptr(prec);  // the links that the operator reads, made on their first use
   // The spare residuals come after everything that the Krylov phase cannot do
-  // without, and go again if they leave the driver no room for the graph; the
-  // refinement gets their memory back (below).
+  // without, and go again if the memory that they take from the device leaves the
+  // driver no room for the graph; the refinement gets theirs back (below).
   std::vector<std::unique_ptr<Field>> rf;
   rf.emplace_back(new Field(prec, n));
   try {
+    const size_t had = pool_reserved();
     while ((int)rf.size() < group) rf.emplace_back(new Field(prec, n));
-    if (group > 1 && !room_beside_pool(MS_SPARE_MARGIN)) throw Error{CPSB_ERR_OOM, "no room beside the spare residuals"};
+    const bool grew = !rf.back()->data.pooled || pool_reserved() != had;
+    if (group > 1 && grew && !room_beside_pool(MS_SPARE_MARGIN)) throw Error{CPSB_ERR_OOM, "no room beside the spare residuals"};
   } catch (const Error &e) {
     if (e.code != CPSB_ERR_OOM) throw;
     rf.resize(1);
@@ -579,7 +581,7 @@ int multishift_multi(Gauge *G, const cpsb_dirac_params &p, const cpsb_cg_arg &a,
       set_capturing(false);
       CK(cudaStreamEndCapture(st, &graph));
       CK(cudaGraphGetNodes(graph, nullptr, &nn));
-      CK(cudaGraphInstantiate(&exec, graph, 0));
+      CK(instantiate_graph(&exec, graph));
       cudaGraphDestroy(graph);
     }
     struct ExecGuard {

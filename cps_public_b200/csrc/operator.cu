@@ -142,6 +142,33 @@ bool room_beside_pool(size_t bytes) {
   return fr >= bytes;
 }
 
+size_t pool_reserved() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  std::lock_guard<std::mutex> lk(pool_mu);
+  auto it = pools().find(dev);
+  unsigned long long n = 0;
+  if (it == pools().end() || !it->second ||
+      cudaMemPoolGetAttribute(it->second, cudaMemPoolAttrReservedMemCurrent, &n) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return (size_t)n;
+}
+
+cudaError_t instantiate_graph(cudaGraphExec_t *exec, cudaGraph_t graph) {
+  cudaError_t e = cudaGraphInstantiate(exec, graph, 0);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    trim_pool();
+    e = cudaGraphInstantiate(exec, graph, 0);
+  }
+  return e;
+}
+
 DevBuf::DevBuf(size_t n) { alloc(n); }
 void DevBuf::release() {
   if (!p) return;

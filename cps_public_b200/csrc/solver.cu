@@ -141,7 +141,7 @@ void CgSolver::run_batches(int batch, cudaStream_t st, const bool *done, bool an
       set_capturing(false);
       CK(cudaStreamEndCapture(st, &g));
       CK(cudaGraphGetNodes(g, nullptr, &nn));
-      CK(cudaGraphInstantiate(&graph, g, 0));
+      CK(instantiate_graph(&graph, g));
       cudaGraphDestroy(g);
     }
     graph_nodes = nn;
